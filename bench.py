@@ -241,7 +241,7 @@ def run_ours(args) -> None:
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record(stream)
         kern.compute_pairfree_device(db, npv_d, bmax, TAU, p0, p1 - p0, matrix=True,
-                                     out=out)                       # 3 launches
+                                     out=out)                       # 5 launches
         if record_te:
             e1.record(stream)
             te_times.append((e0, e1))
@@ -382,7 +382,8 @@ def run_ours(args) -> None:
                        "pairs": total, "step": "remap + coarsen + all-pairs TE matrix",
                        "parallelism": f"pair-range x{world}", "l2": "inputs (200 MB) > L2",
                        "launch": kern.cfg, "launch_resolved": launch_resolved},
-            "gpu_launches": 6 * args.steps,  # remap, coarsen x2, prepass, order, TE tile
+            # remap, coarsen x2, prepass, plan, planes, tensor-core TE, TE tile
+            "gpu_launches": 8 * args.steps,
             "roofline": roofline, "roofline_hbm": roofline_hbm,
             "cpu_baseline": cpu, "e2e": e2e, "clocks": clk.summary(), "surrogate": sur,
             "binary_path": binl, "fdr": fdrl, "cfg3": c3, "cfg1": c1, "next_rows": nxt,

@@ -75,13 +75,20 @@ int tenex_last_error(char* buf, size_t len);
  * query_smem_optin helper (tenex/kernels/__init__.py:44-71). */
 int tenex_device_query(int device, tenex_dev_info* info);
 
-/* Bytes of device workspace the TE / surrogate entry points need: a 256-byte
- * header (work tickets, validation words) plus the source processing order
- * (n_vars int32, genes sorted by bin count), rounded up to 256 bytes; plus, when
- * pairs with b up to b_max would not fit a shared-memory slot on the current
- * device (coarsening off), the global-memory histogram slots of the overflow
- * launch. A workspace without them makes such a call fail with the size it
- * needs. */
+/* Bytes of device workspace the pair-list entry points need, and the least the
+ * other TE / surrogate entry points accept: a 256-byte header (work tickets,
+ * validation words) plus the source processing order (n_vars int32, genes sorted
+ * by bin count), rounded up to 256 bytes; plus, when pairs with b up to b_max
+ * would not fit a shared-memory slot on the current device (coarsening off), the
+ * global-memory histogram slots of the overflow launch. A workspace without them
+ * makes such a call fail with the size it needs. */
+size_t tenex_te_pairs_workspace_bytes(int n_vars, int64_t row_len, int b_max);
+
+/* The same plus room for the tensor-core histograms of the all-pairs entry points:
+ * tables (about 5 KB a gene) and bit planes (row_len / 4 bytes for each of a gene's
+ * bins up to 16, at most 8 GiB). With a smaller workspace (256-byte aligned, at
+ * least tenex_te_pairs_workspace_bytes) they use what fits, down to none: every
+ * pair then runs in the shared-memory kernel. */
 size_t tenex_te_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 
 /* The launch shape the histogram kernels would use on the current device for

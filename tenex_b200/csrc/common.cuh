@@ -37,12 +37,15 @@ __host__ __device__ inline int64_t round_up(int64_t x, int64_t m) { return (x + 
 //   [4]   int32  data-validation word (nonzero = bad bin / n_per_var)
 //   [8]   int32  unsupported-item word (nonzero = an item's histogram did not fit)
 //   [12]  uint32 work ticket of the global-memory overflow launch
+//   [16]  sizes of the tensor-core launch's plan: work items, blocks of source tiles,
+//         source tiles
 struct WsHeader {
   unsigned int ticket;
   int bad_data;
   int bad_item;
   unsigned int ov_ticket;
-  int pad[60];
+  int mma_items, mma_blocks, mma_stiles;
+  int pad[57];
 };
 static_assert(sizeof(WsHeader) == 256, "workspace header is 256 bytes");
 

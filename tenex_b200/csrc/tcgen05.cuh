@@ -162,5 +162,80 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
       : "memory");
 }
 
+// ---- CTA pairs (clusters of 2, cta_group::2) --------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+// Barrier over every thread of the cluster (release / acquire).
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Arrival on the same barrier of the cluster's CTA `cta` (which may be this one).
+__device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(bar)), "r"(cta));
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(a) : "memory");
+}
+
+// mbar_wait for a barrier that the other CTA of the cluster arrives on too.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
+  const uint32_t a = smem_u32(bar);
+  for (uint32_t it = 0; it < kSpinLimit; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
+// mma_mxf4 over a CTA pair: M = 256 rows, each CTA's half of A's rows and of B's
+// columns from its own shared memory, each CTA's 128 rows of D in its own TMEM.
+// Issued by the even CTA only; the TMEM addresses are the same in both. a and b are
+// the low words of smem_desc_sw128 descriptors (the high word is a constant), sf the
+// unit scale factors of both operands.
+__device__ __forceinline__ void mma_mxf4_pair(uint32_t d_tmem, uint32_t a, uint32_t b,
+                                              uint32_t idesc, uint32_t accumulate, uint32_t sf) {
+  constexpr uint32_t kHigh = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO, version, swizzle
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 ad, {%1, %6};\n\t"
+      "mov.b64 bd, {%2, %6};\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], ad, bd, %3, [%5], [%5], "
+      "p;\n\t}" ::"r"(d_tmem),
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(sf), "r"(kHigh)
+      : "memory");
+}
+
+// One arrival on `bar` of both CTAs once every MMA issued before has completed.
+__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
+      "[%0], %1;" ::"r"(smem_u32(bar)),
+      "h"((unsigned short)3)
+      : "memory");
+}
 
 }  // namespace tenex

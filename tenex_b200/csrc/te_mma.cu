@@ -1,0 +1,966 @@
+// te_mma.cu — joint histograms of many (source, target) pairs as one contraction on
+// the tensor cores, for pairs whose histogram has few cells.
+//
+// The counts c3[xt1, xt, y] of a pair are inner products over the samples of two 0/1
+// vectors: [x[s+lag] = xt1 and x[s] = xt] of the target and [y[s] = y] of the source.
+// So the histograms of all pairs are one matrix product: rows = (source, y), columns
+// = (target, occupied state (xt1, xt)), K = samples. It costs one multiply-add per
+// cell and sample where counting costs one shared-memory reduction per sample
+// (2.2e12 of them per second), so pairs of up to kMaxCells cells come here and the
+// others stay with te_pair.cu. Measured, all pairs, counting alone -> with this path:
+// 10,000 genes x 20,000 samples (b to 16, 5% to 38) 928 -> 705 ms, 2,000 x 5,000
+// (b to 16) 11.3 -> 8.6 ms, 3,281 x 458 (b to 7, every pair here) 7.1 -> 2.2 ms,
+// 301 x 101,003 (b to 12) 6.1 -> 3.4 ms.
+//
+//   * plan (one CTA): sources sorted by bin count and targets by occupied states are
+//     cut into tiles of at most 128 rows and 240 columns, whole genes only, so a
+//     pair's cells lie in one tile. Which pairs come here depends on the pair alone
+//     (columns of the target x bins of the source), not on the tiles.
+//   * planes: one bit per (gene, bin, sample), of x and of x shifted by the lag, the
+//     shifted one so that the words of a column are an AND of two aligned words.
+//   * contraction: eight warps expand 256 samples of a tile's rows and columns at a
+//     time from bits to packed E2M1 values in shared memory (four bit positions of a
+//     word go to the four words of a 16-byte chunk, as 0.5, 1 or 2, the other operand
+//     scaled inversely so every product is 1: no shifting of single bits); a ninth
+//     issues tcgen05.mma kind::mxf4 with unit block scales into 240 float32 TMEM
+//     columns (whole numbers, exact below 2^24). From HBM and L2 come 1 bit per row
+//     and sample, not 4: 1.4 KB per 64 samples and tile instead of 12 KB, which L2
+//     could not deliver.
+//   * epilogue: a TMEM lane is one (source, y); it walks the columns of each target by
+//     xt, so c2b is a sum of its own registers. The terms are te_pair.cu's, operation
+//     for operation; sums over xt1 are float32, over xt and y float64.
+//   * Bound: the producers. A 256-sample step of a 256 x 240 tile takes a CTA pair
+//     about 1,100 cycles with two pairs on the SMs' shared-memory and logic pipes; its
+//     MMAs alone take under 400 (measured with operands left as they were).
+//   * Two CTAs share an SM (256 TMEM columns each): one's epilogue runs under the
+//     other's contraction. Work items go round the CTA pairs in an order that takes 16
+//     source tiles at a time across all target tiles, so the planes in use stay in L2.
+//   * Every mbarrier wait is bounded; on expiry the kernel sets the workspace's item
+//     word and leaves after freeing its TMEM.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "te_mma.cuh"
+#include "tcgen05.cuh"
+
+namespace tenex {
+namespace {
+
+constexpr int kMaxCells = 1200;   // occupied target states x source bins of a pair
+constexpr int kMaxTgtBins = 16;   // target bins (at most 16 columns share an xt)
+constexpr int kMaxCols = 240;     // columns of a tile
+constexpr int kRows = 128;        // rows of a tile (TMEM lanes) per CTA of a pair
+constexpr int kMaxSrcBins = 64;   // source bins
+constexpr int kBlk = 8;           // pairs of source tiles per block of the item order
+constexpr int kStages = 3;
+constexpr int kABytes = kRows * 128, kBBytes = kMaxCols / 2 * 128;
+constexpr int kStageBytes = kABytes + kBBytes;
+constexpr int kProducers = 256;   // threads that expand operands and run the epilogue
+constexpr int kThreads = kProducers + 32;
+constexpr uint32_t kSfCol = 248;  // TMEM columns of the unit scale factors
+constexpr int kTmemCols = 256;
+// Partial sums of a tile: one float64 row of kRows per target, two for targets of
+// kSplitCols columns or more (those of kSplitBins bins or more, which have at least
+// kSplitBins - 1 columns, are summed by two warps per lane quarter).
+constexpr int kSlots = 60, kSplitCols = 7, kSplitBins = 8;
+constexpr int kBlkCache = 128;    // item blocks whose starts sit in shared memory
+static_assert(kSlots * kRows * 8 <= kStages * kStageBytes, "partial sums fit the stages");
+
+// ---------------------------------------------------------------------------
+// Validation and the target states' counts. One CTA per gene: every bin of gene g
+// in [0, row_len) below n_per_var[g] and 1 <= n_per_var[g] <= b_max, else
+// ws->bad_data. Targets of few bins also get c2a and the number of occupied states.
+__global__ void __launch_bounds__(256) gene_prepass_kernel(TeMma M) {
+  __shared__ int h[256];
+  const int g = blockIdx.x, tid = threadIdx.x;
+  const int b = M.npv[g];
+  const uint8_t* row = M.bins + (int64_t)g * M.ld;
+  const int64_t nvec = M.row_len >> 4;
+  bool bad = b < 1 || b > M.b_max;
+  const uint4* rv = reinterpret_cast<const uint4*>(row);
+  for (int64_t v = tid; v < nvec; v += blockDim.x) {
+    const uint4 q = __ldg(rv + v);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int bb = 0; bb < 4; ++bb) bad |= ((w[k] >> (8 * bb)) & 0xffu) >= (uint32_t)b;
+  }
+  for (int64_t i = (nvec << 4) + tid; i < M.row_len; i += blockDim.x) bad |= row[i] >= b;
+  if (__syncthreads_or(bad)) {
+    if (tid == 0) atomicExch(&M.ws->bad_data, 1);
+    return;
+  }
+  if (M.cap_rows == 0) return;
+  if (b > kMaxTgtBins || g < M.t_first || g > M.t_last) {
+    if (tid == 0) M.ncols[g] = 0;
+    return;
+  }
+  h[tid] = 0;
+  __syncthreads();
+  // four samples per step: an aligned word of x[s] and the two words around x[s + lag]
+  const uint32_t* rw = reinterpret_cast<const uint32_t*>(row);
+  const int last = (int)(M.ld >> 2) - 1, sh = (M.lag & 3) * 8;
+  for (int s = tid * 4; s < M.N; s += 256 * 4) {
+    const uint32_t a = __ldg(rw + (s >> 2));
+    const int w1 = (s + M.lag) >> 2;
+    const uint32_t c = __funnelshift_r(__ldg(rw + w1), __ldg(rw + min(w1 + 1, last)), sh);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (s + u < M.N)
+        atomicAdd(&h[((c >> (8 * u)) & 0xffu) * (uint32_t)b + ((a >> (8 * u)) & 0xffu)], 1);
+  }
+  __syncthreads();
+  const int v = h[tid];
+  M.c2a[(int64_t)g * 256 + tid] = v;
+  const int occ = __syncthreads_count(v > 0);
+  if (tid == 0) M.ncols[g] = occ <= kMaxCols ? occ : 0;
+}
+
+// ---------------------------------------------------------------------------
+// Plan: one CTA of 1024 threads.
+struct PlanShared {
+  int cnt[256], base[256], width[256], scan[256];
+  int wc[32][256];
+  int cls[256], n_cls;                       // classes with members, ascending
+  int seg_tile[256], seg_pos[256], seg_per[256], seg_n[256], n_seg;
+  int open_tile[256], open_pos[256], open_n[256], n_open;
+  int n_tiles, n_src;
+};
+
+// Exclusive prefix sums of a[0..255] into out (all threads call).
+__device__ void scan256(const int* a, int* out, int* tmp, int tid) {
+  if (tid < 256) tmp[tid] = a[tid];
+  __syncthreads();
+  for (int o = 1; o < 256; o <<= 1) {
+    const int v = (tid < 256 && tid >= o) ? tmp[tid - o] : 0;
+    __syncthreads();
+    if (tid < 256) tmp[tid] += v;
+    __syncthreads();
+  }
+  if (tid < 256) out[tid] = tmp[tid] - a[tid];
+  __syncthreads();
+}
+
+// Stable counting sort of 0..n-1 by key(g) in 0..255 into `order`; leaves the class
+// sizes in S.cnt and the class starts in S.base.
+template <class Key>
+__device__ void stable_order(PlanShared& S, int n, Key key, int32_t* order, int tid) {
+  const int lane = tid & 31, w = tid >> 5;
+  if (tid < 256) S.cnt[tid] = 0;
+  __syncthreads();
+  for (int g = tid; g < n; g += 1024) atomicAdd(&S.cnt[key(g)], 1);
+  __syncthreads();
+  scan256(S.cnt, S.base, S.scan, tid);
+  if (tid < 256) S.scan[tid] = S.base[tid];  // next free position of each class
+  for (int start = 0; start < n; start += 1024) {
+    for (int i = tid; i < 32 * 256; i += 1024) (&S.wc[0][0])[i] = 0;
+    __syncthreads();
+    const int g = start + tid;
+    const bool in = g < n;
+    const int k = in ? key(g) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, k);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    if (in && rank == 0) S.wc[w][k] = __popc(same);
+    __syncthreads();
+    if (tid < 256) {
+      int run = S.scan[tid];
+#pragma unroll 8
+      for (int ww = 0; ww < 32; ++ww) {
+        const int c = S.wc[ww][tid];
+        S.wc[ww][tid] = run;
+        run += c;
+      }
+      S.scan[tid] = run;
+    }
+    __syncthreads();
+    if (in) order[S.wc[w][k] + rank] = g;
+    __syncthreads();
+  }
+}
+
+// Cuts the sorted positions of classes [c_lo, c_hi] (class = width of a member) into
+// tiles of at most `room` width and `most` members (a member of a class from `dbl` on
+// counts twice), positions from `limit` on left out. Full tiles of one class come out as segments (emitted in parallel by
+// emit_tiles), those that span classes one by one.
+__device__ void pack_tiles(PlanShared& S, int c_lo, int c_hi, int room, int most, int dbl,
+                           int limit, int tid) {
+  if (tid == 0) {
+    S.n_seg = S.n_open = 0;
+    int tile = 0, k = 0, used = 0, weight = 0, pos0 = 0;
+    for (int ci = 0; ci < S.n_cls; ++ci) {
+      const int c = S.cls[ci];
+      if (c < c_lo || c > c_hi) continue;
+      int pos = S.base[c];
+      int m = min(S.cnt[c], limit - pos);
+      if (m <= 0) break;
+      const int wt = c >= dbl ? 2 : 1;
+      const int per = min(room / c, most / wt);
+      if (k > 0) {
+        const int r = min(m, min((room - used) / c, (most - weight) / wt));
+        k += r;
+        used += r * c;
+        weight += r * wt;
+        pos += r;
+        m -= r;
+        if (m > 0) {
+          S.open_tile[S.n_open] = tile++;
+          S.open_pos[S.n_open] = pos0;
+          S.open_n[S.n_open++] = k;
+          k = 0;
+        }
+      }
+      if (m > 0) {
+        const int f = m / per;
+        S.seg_tile[S.n_seg] = tile;
+        S.seg_pos[S.n_seg] = pos;
+        S.seg_per[S.n_seg] = per;
+        S.seg_n[S.n_seg++] = f;
+        tile += f;
+        pos += f * per;
+        m -= f * per;
+        if (m > 0) {
+          pos0 = pos;
+          k = m;
+          used = m * c;
+          weight = m * wt;
+        }
+      }
+    }
+    if (k > 0) {
+      S.open_tile[S.n_open] = tile++;
+      S.open_pos[S.n_open] = pos0;
+      S.open_n[S.n_open++] = k;
+    }
+    S.n_tiles = tile;
+  }
+  __syncthreads();
+}
+
+template <class Emit>
+__device__ void emit_tiles(const PlanShared& S, Emit emit, int tid) {
+  for (int i = tid; i < S.n_open; i += 1024) emit(S.open_tile[i], S.open_pos[i], S.open_n[i]);
+  for (int s = tid >> 5; s < S.n_seg; s += 32)
+    for (int i = tid & 31; i < S.seg_n[s]; i += 32)
+      emit(S.seg_tile[s] + i, S.seg_pos[s] + i * S.seg_per[s], S.seg_per[s]);
+  __syncthreads();
+}
+
+__device__ void list_classes(PlanShared& S, int tid) {
+  if (tid < 256) S.width[tid] = S.cnt[tid] > 0;
+  __syncthreads();
+  scan256(S.width, S.cls, S.scan, tid);
+  const int at = tid < 256 ? S.cls[tid] : 0;
+  __syncthreads();
+  if (tid < 256 && S.width[tid]) S.cls[at] = tid;
+  if (tid == 255) S.n_cls = at + S.width[255];
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(1024) plan_kernel(TeMma M) {
+  __shared__ PlanShared S;
+  const int tid = threadIdx.x, n = M.n;
+  // bins already found invalid: the launches that follow do nothing. (Counts outside
+  // 1..255 stay in bounds here.)
+  const bool bad = *(volatile int*)&M.ws->bad_data != 0;
+  stable_order(S, n, [&](int g) { return min(max(M.npv[g], 0), 255); }, M.order, tid);
+  if (M.cap_rows == 0 || bad) return;
+  list_classes(S, tid);
+  // plane rows by position: class start + rank x bins, as far as there is room
+  if (tid < 256) S.width[tid] = tid <= kMaxSrcBins ? S.cnt[tid] * tid : 0;
+  __syncthreads();
+  scan256(S.width, S.wc[0], S.scan, tid);
+  if (tid == 0) {
+    int pos = 0;
+    for (int ci = 0; ci < S.n_cls; ++ci) {
+      const int c = S.cls[ci];
+      if (c < 1 || c > kMaxSrcBins) break;
+      const int64_t fit = (M.cap_rows - S.wc[0][c]) / c;
+      if (fit <= 0) break;
+      pos = S.base[c] + (int)(fit < S.cnt[c] ? fit : S.cnt[c]);
+      if (fit < S.cnt[c]) break;
+    }
+    S.n_src = pos;
+  }
+  __syncthreads();
+  const int n_src = S.n_src;
+  for (int pos = tid; pos < n; pos += 1024) {
+    const int g = M.order[pos], c = M.npv[g];
+    const int row = pos < n_src ? S.wc[0][c] + (pos - S.base[c]) * c : -1;
+    M.rowoff[g] = row;
+    M.src[pos] = make_int2(g, row);
+  }
+  pack_tiles(S, 1, kMaxSrcBins, kRows, kRows, 256, n_src, tid);
+  emit_tiles(S, [&](int t, int pos, int m) {
+    const int2 a = M.src[pos], b = M.src[pos + m - 1];
+    M.stile[t] = make_int4(pos, m, a.y, b.y + M.npv[b.x] - a.y);
+  }, tid);
+  const int n_stiles = S.n_tiles;
+  // how many source positions each target takes: those with bins x columns within
+  // kMaxCells (S.base still holds the sources' class starts)
+  for (int g = tid; g < n; g += 1024) {
+    int nc = M.ncols[g], cut = 0;
+    if (M.rowoff[g] < 0) nc = 0;
+    if (nc > 0) {
+      const int c = kMaxCells / nc;
+      cut = min(c >= 255 ? n : S.base[c + 1], n_src);
+      if (cut == 0) nc = 0;
+    }
+    M.ncols[g] = nc;
+    M.cut[g] = cut;
+  }
+  __syncthreads();
+  stable_order(S, n, [&](int g) { return M.ncols[g]; }, M.torder, tid);
+  list_classes(S, tid);
+  if (tid < 256) S.width[tid] = S.cnt[tid] * tid;
+  __syncthreads();
+  scan256(S.width, S.wc[0], S.scan, tid);
+  for (int pos = tid; pos < n; pos += 1024) {
+    const int g = M.torder[pos], c = M.ncols[g];
+    M.tpos[g] = pos;
+    M.tgt[pos] = make_int4(g, M.npv[g], S.wc[0][c] + (pos - S.base[c]) * c, M.cut[g]);
+  }
+  pack_tiles(S, 1, kMaxCols, kMaxCols, kSlots, kSplitCols, n, tid);
+  emit_tiles(S, [&](int t, int pos, int m) {
+    const int4 a = M.tgt[pos], b = M.tgt[pos + m - 1];
+    M.ttile[t] = make_int4(pos, m, a.z, b.z + M.ncols[b.x] - a.z);
+    // the tile's first target has the fewest columns, so the most sources
+    const int cut = a.w;
+    int lo = 0, hi = n_stiles;  // source tiles that start below cut
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (M.stile[mid].x < cut) lo = mid + 1;
+      else hi = mid;
+    }
+    M.nst[t] = lo;
+  }, tid);
+  const int n_ttiles = S.n_tiles;
+  // items: block by block of kBlk pairs of source tiles, within it target tile by
+  // target tile
+  const int n_pairs = (n_stiles + 1) / 2, n_blk = (n_pairs + kBlk - 1) / kBlk;
+  int run = 0;
+  for (int b0 = 0; b0 < n_blk; b0 += 256) {
+    const int b = b0 + tid;
+    if (tid < 256) {
+      int lo = 0, hi = n_ttiles;  // target tiles that reach into the block (nst descends)
+      if (b < n_blk)
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (M.nst[mid] > b * kBlk * 2) lo = mid + 1;
+          else hi = mid;
+        }
+      S.width[tid] = b < n_blk ? lo * min(kBlk, n_pairs - b * kBlk) : 0;
+    }
+    __syncthreads();
+    scan256(S.width, S.cls, S.scan, tid);
+    if (tid < 256 && b <= n_blk) M.blk[b] = run + S.cls[tid];
+    run += S.cls[255] + S.width[255];
+    __syncthreads();
+  }
+  if (tid == 0) {
+    M.blk[n_blk] = run;
+    M.ws->mma_blocks = n_blk;
+    M.ws->mma_stiles = n_stiles;
+    M.ws->mma_items = run;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Bit planes of a gene (one warp per 256 samples) and a target's column table.
+__global__ void __launch_bounds__(256) planes_kernel(TeMma M) {
+  if (*(volatile int*)&M.ws->bad_data != 0) return;
+  const int g = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row0 = M.rowoff[g];
+  if (row0 < 0) return;
+  const int b = M.npv[g], nc = M.ncols[g];
+  const uint8_t* row = M.bins + (int64_t)g * M.ld;
+  const int n_blocks = M.words >> 3;
+  for (int kb = blockIdx.y * 8 + warp; kb < n_blocks; kb += gridDim.y * 8) {
+    uint32_t x0[8], x1[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int64_t s = (int64_t)kb * 256 + k * 32 + lane;
+      x0[k] = s < M.row_len ? row[s] : 255u;
+      x1[k] = nc > 0 && s + M.lag < M.row_len ? row[s + M.lag] : 255u;
+    }
+    for (int v0 = 0; v0 < b; v0 += 32) {
+      uint32_t p[8] = {}, f[8] = {};
+      const int vn = min(32, b - v0);
+      for (int v = 0; v < vn; ++v) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t m = __ballot_sync(0xffffffffu, x0[k] == (uint32_t)(v0 + v));
+          if (lane == v) p[k] = m;
+        }
+        if (nc > 0)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const uint32_t m = __ballot_sync(0xffffffffu, x1[k] == (uint32_t)(v0 + v));
+            if (lane == v) f[k] = m;
+          }
+      }
+      if (lane < vn) {
+        const int64_t at = (kb * M.cap_rows + row0 + v0 + lane) * 8;
+        uint4* d = reinterpret_cast<uint4*>(M.P + at);
+        d[0] = make_uint4(p[0], p[1], p[2], p[3]);
+        d[1] = make_uint4(p[4], p[5], p[6], p[7]);
+        if (nc > 0) {
+          d = reinterpret_cast<uint4*>(M.F + at);
+          d[0] = make_uint4(f[0], f[1], f[2], f[3]);
+          d[1] = make_uint4(f[4], f[5], f[6], f[7]);
+        }
+      }
+    }
+  }
+  // columns by x_t = j, then x_{t+lag} = i, occupied states only
+  if (nc > 0 && blockIdx.y == 0 && warp == 0) {
+    const int32_t* c2a = M.c2a + (int64_t)g * 256;
+    int occ = 0, c1 = 0;
+    if (lane < b)
+      for (int i = 0; i < b; ++i) {
+        const int c = c2a[i * b + lane];
+        occ += c > 0;
+        c1 += c;
+      }
+    int at = occ;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += t;
+    }
+    at -= occ;
+    if (lane < b) {
+      const int pos = M.tpos[g], c0 = M.tgt[pos].z;
+      M.grp[(int64_t)pos * 16 + lane] = (uint32_t)c1 | ((uint32_t)occ << 24);
+      for (int i = 0; i < b; ++i) {
+        const int c = c2a[i * b + lane];
+        if (c == 0) continue;
+        M.colq[c0 + at] = make_float2(__fdiv_rn((float)c1, (float)c), (float)c);
+        M.colrow[c0 + at] = make_int2(row0 + i, row0 + lane);
+        ++at;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The contraction.
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+        "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// 32 samples of a row (source) or a column (target) as E2M1 values: bit position
+// 4 i + j goes to nibble i of word j, with the values 0.5, 1, 2, 1 (rows) and
+// 2, 1, 0.5, 1 (columns) for j = 0..3.
+__device__ __forceinline__ uint4 expand_row(uint32_t m) {
+  return make_uint4(m & 0x11111111u, m & 0x22222222u, m & 0x44444444u, (m >> 2) & 0x22222222u);
+}
+__device__ __forceinline__ uint4 expand_col(uint32_t m) {
+  const uint32_t d = m >> 2;
+  return make_uint4((m << 2) & 0x44444444u, m & 0x22222222u, d & 0x11111111u, d & 0x22222222u);
+}
+
+// Sum over the L states xt1 of one xt (this lane's source bin y) of te_pair.cu's
+// terms: c log2(c (1 / c2b) (c1 / c2a)), exactly 0 where c c1 == c2a c2b. An empty
+// cell has a ratio of 0 (or, in an empty column, a NaN: fmaxf returns the other
+// operand), so its term is 0 times a finite logarithm.
+template <int L, int R>
+__device__ __forceinline__ float group_terms(const uint32_t (&r)[R], const float2* q, float c1) {
+  float b = 0.f;
+#pragma unroll
+  for (int u = 0; u < L; ++u) b += __uint_as_float(r[u]);
+  const float inv = __frcp_rn(fmaxf(b, 1.f));
+  float acc = 0.f;
+#pragma unroll
+  for (int u = 0; u < L; ++u) {
+    const float c = __uint_as_float(r[u]);
+    const float2 qu = q[u];
+    const float x = fmaxf(c * inv * qu.x, 1e-30f);
+    float t;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
+    const float with = fmaf(c, t, acc);
+    acc = c * c1 == qu.y * b ? acc : with;
+  }
+  return acc;
+}
+
+__device__ __forceinline__ float group_sum(uint32_t taddr, int len, const float2* q, float c1) {
+  if (len <= 8) {
+    uint32_t r[8];
+    tmem_ld(taddr, r);
+    switch (len) {
+      case 1: return group_terms<1>(r, q, c1);
+      case 2: return group_terms<2>(r, q, c1);
+      case 3: return group_terms<3>(r, q, c1);
+      case 4: return group_terms<4>(r, q, c1);
+      case 5: return group_terms<5>(r, q, c1);
+      case 6: return group_terms<6>(r, q, c1);
+      case 7: return group_terms<7>(r, q, c1);
+      default: return group_terms<8>(r, q, c1);
+    }
+  }
+  uint32_t r[16];
+  tmem_ld(taddr, r);
+  switch (len) {
+    case 9: return group_terms<9>(r, q, c1);
+    case 10: return group_terms<10>(r, q, c1);
+    case 11: return group_terms<11>(r, q, c1);
+    case 12: return group_terms<12>(r, q, c1);
+    case 13: return group_terms<13>(r, q, c1);
+    case 14: return group_terms<14>(r, q, c1);
+    case 15: return group_terms<15>(r, q, c1);
+    default: return group_terms<16>(r, q, c1);
+  }
+}
+
+// A work item's tables, copied from global memory while the item before it is in its
+// epilogue.
+struct Tables {
+  int4 st, tt;           // M.stile (of this CTA's half), M.ttile; st.x < 0 ends the launch
+  int wide0;             // first target of kSplitCols columns or more (targets ascend)
+  float2 q[kMaxCols];    // M.colq
+  int2 row[kMaxCols / 2];     // M.colrow of the columns this CTA expands
+  uint32_t grp[kSlots * 16];  // M.grp
+  int4 tgt[kSlots];      // M.tgt
+  int2 src[kRows + 1];   // gene, first row in the tile; then the number of rows
+};
+
+struct Shared {
+  Tables tab[2];
+  int blk[kBlkCache];
+  uint64_t full[kStages], empty[kStages], acc;
+  uint32_t tmem;
+  int abort;
+};
+constexpr int kSmemBytes = kStages * kStageBytes + 1024 + (int)sizeof(Shared);
+static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs share an SM");
+
+// Four words of bits as four 16-byte chunks (half a step) of an operand row at `row`,
+// chunk c at ((c * 16) ^ sw): the 128-byte swizzle.
+template <bool ROW>
+__device__ __forceinline__ void put_half(unsigned char* row, uint32_t sw, const uint32_t (&m)[4]) {
+#pragma unroll
+  for (uint32_t c = 0; c < 4; ++c)
+    *reinterpret_cast<uint4*>(row + ((c << 4) ^ sw)) = ROW ? expand_row(m[c]) : expand_col(m[c]);
+}
+
+// Fills T for the next item with work, from item number q on in steps of the number
+// of CTA pairs (one warp). Both CTAs of a pair walk the same numbers.
+__device__ void next_item(const TeMma& M, Shared& S, Tables& T, uint32_t* q_io, uint32_t rank,
+                          int n_items, int n_blk, int n_stiles, int lane) {
+  const int* blk = n_blk <= kBlkCache ? S.blk : M.blk;
+  const int n_pairs = (n_stiles + 1) / 2;
+  uint32_t q = *q_io;
+  int i = -1, j = 0;
+  for (; q < (uint32_t)n_items; q += gridDim.x >> 1) {
+    int lo = 0, hi = n_blk - 1;  // last block that starts at or below q
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (blk[mid] <= (int)q) lo = mid;
+      else hi = mid - 1;
+    }
+    const int w = min(kBlk, n_pairs - lo * kBlk), rem = (int)q - blk[lo];
+    j = rem / w;
+    const int i0 = (lo * kBlk + rem - j * w) * 2;
+    if (i0 < M.nst[j]) {
+      i = i0 + (int)rank;
+      q += gridDim.x >> 1;
+      break;
+    }
+  }
+  *q_io = q;
+  if (i < 0) {
+    if (lane == 0) T.st.x = -1;
+    return;
+  }
+  const int4 st = i < n_stiles ? M.stile[i] : make_int4(0, 0, 0, 0), tt = M.ttile[j];
+  if (lane == 0) {
+    T.st = st;
+    T.tt = tt;
+    T.src[st.y] = make_int2(0, st.w);
+  }
+  for (int c = lane; c < tt.w; c += 32) T.q[c] = M.colq[tt.z + c];
+  const int n_half = (tt.w + 15) / 16 * 8, c0 = (int)rank * n_half;
+  for (int c = lane; c < n_half && c0 + c < tt.w; c += 32) T.row[c] = M.colrow[tt.z + c0 + c];
+  int narrow = 0;
+  for (int t = lane; t < tt.y; t += 32) {
+    const int4 v = M.tgt[tt.x + t];
+    T.tgt[t] = v;
+    narrow += M.ncols[v.x] < kSplitCols;
+  }
+  narrow = __reduce_add_sync(0xffffffffu, narrow);
+  if (lane == 0) T.wide0 = narrow;
+  for (int k = lane; k < tt.y * 16; k += 32) T.grp[k] = M.grp[(int64_t)tt.x * 16 + k];
+  for (int s = lane; s < st.y; s += 32) {
+    const int2 v = M.src[st.x + s];
+    T.src[s] = make_int2(v.x, v.y - st.z);
+  }
+}
+
+// One pair's TE to the launch's output (one thread per pair).
+__device__ __forceinline__ void put_pair(const TeMma& M, int src, int tgt, double tot) {
+  const int64_t p = (int64_t)tgt * (M.n - 1) + (src < tgt ? src : src - 1);
+  if (src == tgt || p < M.p0 || p >= M.p1) return;
+  const float te = (float)(tot * M.inv_N);
+  if (M.out_mode == kOutPairfree) {
+    M.out[p - M.p0] = te;
+  } else if (M.out_mode == kOutMatrix) {
+    M.out[(int64_t)src * M.out_ld + tgt] = te;
+  } else {
+    const int64_t m = (int64_t)src * M.n + tgt;
+    const double td = (double)te;
+    atomicAdd(M.sum + m, td);
+    atomicAdd(M.sumsq + m, td * td);
+    if (te >= M.obs[m]) atomicAdd(M.cnt_ge + m, 1);
+  }
+}
+
+// Raw counts of this lane's (source, y) for target tt (parity checks only).
+__device__ void put_counts(const TeMma& M, const Tables& T, int tt, int row, uint32_t lane_base) {
+  int s = 0;
+  while (s < T.st.y && T.src[s + 1].y <= row) ++s;
+  const bool mine = s < T.st.y;
+  const int4 t = T.tgt[tt];
+  const int src = mine ? T.src[s].x : 0, tgt = t.x, bt = t.y;
+  const int64_t p = (int64_t)tgt * (M.n - 1) + (src < tgt ? src : src - 1);
+  const int bs = mine ? T.src[s + 1].y - T.src[s].y : 1, y = mine ? row - T.src[s].y : 0;
+  const bool put = mine && src != tgt && p >= M.p0 && p < M.p1;
+  int32_t* cd = M.counts_dbg + (put ? (p - M.p0) * M.counts_stride : 0);
+  if (put)
+    for (int z = 0; z < bt * bt; ++z) cd[z * bs + y] = 0;
+  const int r0 = M.rowoff[tgt], c0 = t.z - T.tt.z, nc = M.ncols[tgt];
+  for (int c = 0; c < nc; ++c) {
+    uint32_t r[8];
+    tmem_ld(lane_base + (uint32_t)(c0 + c), r);
+    const int2 cr = M.colrow[t.z + c];
+    if (put) cd[((cr.x - r0) * bt + cr.y - r0) * bs + y] = (int32_t)__uint_as_float(r[0]);
+  }
+}
+
+// Two CTAs (a pair of SMs) share an item: 256 rows, each CTA's own 128 in its TMEM;
+// each expands half of the columns and the even one issues for both
+// (cta_group::2), so a column is expanded once per 256 rows. 10,000 x 20,000: 245 ms,
+// against 315 ms with one CTA per 128-row tile.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_kernel(TeMma M) {
+  if (*(volatile int*)&M.ws->bad_data != 0) return;
+  const int n_items = M.ws->mma_items, n_blk = M.ws->mma_blocks, n_stiles = M.ws->mma_stiles;
+  if (n_items == 0) return;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* stages = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  Shared& S = *reinterpret_cast<Shared*>(stages + kStages * kStageBytes);
+  double* part = reinterpret_cast<double*>(stages);  // [slot][row], epilogue only
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_rank();
+  const int n_steps = (M.N + 255) >> 8;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      // the issuing CTA's: one more arrival for the other CTA's half
+      mbar_init(&S.full[s], kProducers / 32 + (rank == 0 ? 1 : 0));
+      mbar_init(&S.empty[s], 1);
+    }
+    mbar_init(&S.acc, 1);
+    S.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = tid; i < n_blk && n_blk <= kBlkCache; i += kThreads) S.blk[i] = M.blk[i];
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&S.tmem)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  uint32_t q = blockIdx.x >> 1;  // next item number (last warp)
+  if (warp == kProducers / 32)
+    next_item(M, S, S.tab[0], &q, rank, n_items, n_blk, n_stiles, lane);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = S.tmem;
+  if (warp < 4) tmem_st8(tmem + ((uint32_t)(warp * 32) << 16) + kSfCol, 0x7f7f7f7fu);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_sync();  // both CTAs' barriers and scale factors are in place
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  const bool elected = elect_one();
+  const uint32_t desc0 = (uint32_t)smem_desc_sw128(smem_u32(stages));  // low word
+  uint32_t stage = 0, parity = 0;  // of the item's first step, in the ring of stages
+  for (uint32_t item = 0;; ++item) {
+    const Tables& T = S.tab[item & 1];
+    if (T.st.x < 0) break;
+    const int n_tgts = T.tt.y, n_cols = T.tt.w, n_rows = T.st.w, wide0 = T.wide0;
+    const int n_mma = (n_cols + 15) & ~15;  // columns of the MMAs, half from each CTA
+    if (tid < kProducers) {
+      // ---- producers: lane pairs take half a step each of one row of this CTA's and
+      // of one column of its half. A store phase (eight lanes) covers four rows and both
+      // halves: all 32 banks once. Words for the next step are loaded before this one's
+      // are expanded.
+      const int r = tid >> 1, half = tid & 1;
+      const bool a_on = r < n_rows;
+      const bool b_on = r < (n_mma >> 1) && (int)rank * (n_mma >> 1) + r < n_cols;
+      const int2 cr = b_on ? T.row[r] : make_int2(0, 0);
+      const int64_t stride = M.cap_rows * 2;  // 256 samples on
+      const uint4* pa = reinterpret_cast<const uint4*>(M.P) + (a_on ? T.st.z + r : 0) * 2 + half;
+      const uint4* pf = reinterpret_cast<const uint4*>(M.F) + cr.x * 2 + half;
+      const uint4* pq = reinterpret_cast<const uint4*>(M.P) + cr.y * 2 + half;
+      const uint32_t sw = (uint32_t)((r & 7) ^ (half << 2)) << 4;  // both operands' rows
+      unsigned char* const op = stages + r * 128;
+      uint4 va = __ldg(pa), vf = __ldg(pf), vq = __ldg(pq);
+      uint32_t s = stage, ph = parity ^ 1;  // `empty` starts as if just released
+      for (int k = 0; k < n_steps; ++k) {
+        const uint32_t a[4] = {va.x, va.y, va.z, va.w};
+        const uint32_t b[4] = {vf.x & vq.x, vf.y & vq.y, vf.z & vq.z, vf.w & vq.w};
+        if (k + 1 < n_steps) {
+          pa += stride;
+          pf += stride;
+          pq += stride;
+          va = __ldg(pa);
+          vf = __ldg(pf);
+          vq = __ldg(pq);
+        }
+        if (!mbar_wait(&S.empty[s], ph)) {
+          *(volatile int*)&S.abort = 1;
+          break;
+        }
+        unsigned char* const row = op + s * kStageBytes;
+        if (a_on) put_half<true>(row, sw, a);
+        if (b_on) put_half<false>(row + kABytes, sw, b);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (elected) mbar_arrive(&S.full[s]);
+        if (++s == kStages) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+    } else if (rank == 1) {
+      // ---- tells the issuing CTA of this one's stages (a cluster-wide release by
+      // each producer warp would wait for its loads of the next step) ---------------
+      uint32_t s = stage, ph = parity;
+      for (int k = 0; k < n_steps; ++k) {
+        if (!mbar_wait(&S.full[s], ph)) {
+          *(volatile int*)&S.abort = 1;
+          break;
+        }
+        if (elected) mbar_arrive_cluster(&S.full[s], 0);
+        if (++s == kStages) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+    } else {
+      // ---- MMA issue, for both CTAs. The whole warp runs the loop, so that stage
+      // numbers and descriptors stay in uniform registers; one lane issues -----------
+      const uint32_t idesc = idesc_mxf4(2 * kRows, n_mma);
+      const uint32_t last = (uint32_t)(((M.N & 255) + 63) >> 6);  // MMAs of a short last step
+      uint32_t s = stage, ph = parity;
+      for (int k = 0; k < n_steps; ++k) {
+        if (!mbar_wait_cluster(&S.full[s], ph)) {
+          *(volatile int*)&S.abort = 1;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a = desc0 + s * (kStageBytes >> 4), b = a + (kABytes >> 4);
+        const uint32_t n = (k + 1 < n_steps || last == 0) ? 4u : last;  // 64 samples each
+        if (elected) {
+#pragma unroll
+          for (uint32_t kk = 0; kk < 4; ++kk)
+            if (kk < n)
+              mma_mxf4_pair(tmem, a + 2 * kk, b + 2 * kk, idesc, (k > 0 || kk > 0) ? 1u : 0u,
+                            tmem + kSfCol);
+          mma_commit_pair(&S.empty[s]);
+        }
+        __syncwarp();
+        if (++s == kStages) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+      if (elected) mma_commit_pair(&S.acc);
+      __syncwarp();
+    }
+    // where the next item's steps start in the ring
+    stage += (uint32_t)n_steps % kStages;
+    parity ^= ((uint32_t)n_steps / kStages) & 1;
+    if (stage >= kStages) {
+      stage -= kStages;
+      parity ^= 1;
+    }
+
+    // ---- epilogue: this CTA's rows ---------------------------------------------------
+    if (!mbar_wait_sleep(&S.acc, item & 1, 64)) *(volatile int*)&S.abort = 1;
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (*(volatile int*)&S.abort) break;
+    if (tid < kProducers) {
+      const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+      const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+      if ((warp & 3) * 32 < n_rows) {
+        for (int tt = 0; tt < n_tgts; ++tt) {
+          const int4 t = T.tgt[tt];
+          const int c0 = t.z - T.tt.z, bt = t.y;
+          const int slot = tt < wide0 ? tt : 2 * tt - wide0;
+          // targets of many bins: half of the xt each; the split depends on the target
+          // alone, so a pair's sum does not depend on its tile
+          int j0 = 0, j1 = bt;
+          if (bt >= kSplitBins) {
+            const int mid = (bt + (t.x & 1)) >> 1;
+            j0 = half ? mid : 0;
+            j1 = half ? bt : mid;
+          } else if ((tt & 1) != half) {
+            j1 = 0;
+          }
+          if (j1 > 0) {
+            int at = c0;
+            for (int j = 0; j < j0; ++j) at += T.grp[tt * 16 + j] >> 24;
+            double sum = 0.0;
+            for (int j = j0; j < j1; ++j) {
+              const uint32_t g = T.grp[tt * 16 + j];
+              const int len = g >> 24;
+              if (len > 0)
+                sum += (double)group_sum(lane_base + (uint32_t)at, len, T.q + at,
+                                         (float)(g & 0xffffffu));
+              at += len;
+            }
+            part[(slot + (bt >= kSplitBins ? half : 0)) * kRows + row] = sum;
+          }
+          if (M.counts_dbg != nullptr && half == 0) put_counts(M, T, tt, row, lane_base);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    } else {
+      next_item(M, S, S.tab[(item + 1) & 1], &q, rank, n_items, n_blk, n_stiles, lane);
+    }
+    __syncthreads();
+    const int n_src = T.st.y;
+    for (int i = tid; i < n_src * n_tgts; i += kThreads) {
+      const int tt = i / n_src, s = i - tt * n_src;
+      const int4 t = T.tgt[tt];
+      if (T.st.x + s >= t.w) continue;  // te_pair.cu's pair
+      const double* a = part + (tt < wide0 ? tt : 2 * tt - wide0) * kRows;
+      double tot = 0.0;
+      const int y1 = T.src[s + 1].y;
+      if (t.y >= kSplitBins)
+        for (int y = T.src[s].y; y < y1; ++y) tot += a[y] + a[y + kRows];
+      else
+        for (int y = T.src[s].y; y < y1; ++y) tot += a[y];
+      put_pair(M, T.src[s].x, t.x, tot);
+    }
+    __syncthreads();
+  }
+  // a wait ran out: nothing more is issued; what was issued before completes by itself
+  __syncthreads();
+  if (tid == 0 && S.abort) atomicExch(&M.ws->bad_item, 2);
+  __syncwarp();
+  cluster_sync();  // neither CTA's shared memory or TMEM goes while the other runs
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kTmemCols)
+                 : "memory");
+  }
+}
+
+// Buffers behind the base workspace, each 256-byte aligned.
+int64_t tables_bytes(int n) {
+  const int64_t i = round_up((int64_t)n * 4, 256);
+  return 6 * i + 2 * round_up((int64_t)n * 8, 256) /* src, blk */ +
+         3 * round_up((int64_t)n * 16, 256) /* tgt, stile, ttile */ +
+         round_up((int64_t)n * 1024, 256) /* c2a */ + round_up((int64_t)n * 64, 256) /* grp */;
+}
+
+// Most columns the targets can have: b_max^2 each, at most kMaxCols.
+int64_t col_bound(int n, int b_max) {
+  const int b = std::min(b_max, kMaxTgtBins);
+  return (int64_t)n * std::min(b * b, kMaxCols);
+}
+
+}  // namespace
+
+// Plane rows for every gene up to 16 bins; sources of more bins use what those leave.
+// 8 GiB of planes at most (22,000 genes of 16 bins x 100,000 cells).
+int64_t te_mma_bytes(int n, int64_t row_len, int b_max) {
+  if (row_len >= ((int64_t)1 << 24)) return 0;  // float32 counts are exact below 2^24
+  const int64_t plane = round_up(row_len, 256) / 8 * 2;
+  int64_t rows = (int64_t)n * std::min(b_max, kMaxTgtBins);
+  rows = std::min(rows, ((int64_t)8 << 30) / plane);
+  return tables_bytes(n) + round_up(col_bound(n, b_max) * 16, 256) + 256 + rows * plane;
+}
+
+bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
+  M->cap_rows = 0;
+  if (M->row_len >= ((int64_t)1 << 24)) return false;
+  const int n = M->n;
+  M->words = (int)(round_up(M->row_len, 256) / 32);
+  const int64_t cols = col_bound(n, M->b_max);
+  const int64_t fixed = tables_bytes(n) + round_up(cols * 16, 256) + 256;
+  const int64_t rows = (bytes - fixed) / ((int64_t)M->words * 8);
+  if (bytes < fixed || rows < 2) return false;
+  unsigned char* at = mem;
+  auto take = [&](int64_t b) {
+    unsigned char* p = at;
+    at += round_up(b, 256);
+    return p;
+  };
+  M->rowoff = reinterpret_cast<int32_t*>(take((int64_t)n * 4));
+  M->ncols = reinterpret_cast<int32_t*>(take((int64_t)n * 4));
+  M->torder = reinterpret_cast<int32_t*>(take((int64_t)n * 4));
+  M->tpos = reinterpret_cast<int32_t*>(take((int64_t)n * 4));
+  M->cut = reinterpret_cast<int32_t*>(take((int64_t)n * 4));
+  M->nst = reinterpret_cast<int32_t*>(take((int64_t)n * 4));
+  M->src = reinterpret_cast<int2*>(take((int64_t)n * 8));
+  M->blk = reinterpret_cast<int32_t*>(take((int64_t)n * 8));
+  M->tgt = reinterpret_cast<int4*>(take((int64_t)n * 16));
+  M->stile = reinterpret_cast<int4*>(take((int64_t)n * 16));
+  M->ttile = reinterpret_cast<int4*>(take((int64_t)n * 16));
+  M->c2a = reinterpret_cast<int32_t*>(take((int64_t)n * 1024));
+  M->grp = reinterpret_cast<uint32_t*>(take((int64_t)n * 64));
+  M->colq = reinterpret_cast<float2*>(take(cols * 16));
+  M->colrow = reinterpret_cast<int2*>(M->colq + cols);
+  M->cap_rows = std::min<int64_t>(rows, (int64_t)1 << 29);
+  M->P = reinterpret_cast<uint32_t*>(at);
+  M->F = M->P + M->cap_rows * M->words;
+  return true;
+}
+
+bool te_mma_takes_all(const TeMma& M) {
+  const int64_t b = M.b_max;
+  return b * b <= kMaxCols && b * b * b <= kMaxCells && (int64_t)M.n * b <= M.cap_rows;
+}
+
+int te_mma_launch(const TeMma& M, const DevAttr& A, bool pair_list, cudaStream_t stream) {
+  gene_prepass_kernel<<<M.n, 256, 0, stream>>>(M);
+  int st = check_launch("gene_prepass_kernel");
+  if (st || pair_list) return st;
+  plan_kernel<<<1, 1024, 0, stream>>>(M);
+  if ((st = check_launch("plan_kernel")) || M.cap_rows == 0) return st;
+  // about four 256-sample blocks per warp
+  const int blocks = M.words / 8;
+  planes_kernel<<<dim3((unsigned)M.n, (unsigned)std::max(1, std::min(64, blocks / 32))), 256, 0,
+                  stream>>>(M);
+  if ((st = check_launch("planes_kernel"))) return st;
+  cudaError_t e = cudaFuncSetAttribute(te_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kSmemBytes);
+  if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute");
+  te_mma_kernel<<<A.sm_count / 2 * 4, kThreads, kSmemBytes, stream>>>(M);
+  return check_launch("te_mma_kernel");
+}
+
+}  // namespace tenex

@@ -47,10 +47,9 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "te_mma.cuh"
 
 namespace tenex {
-
-enum { kOutPairfree = 0, kOutMatrix = 1, kOutStats = 2 };
 
 struct TeParams {
   const uint8_t* bins;
@@ -97,6 +96,9 @@ struct TeParams {
   int32_t* counts_dbg;
   int64_t counts_stride;
   const int32_t* order; // (n,) genes stably sorted by bin-count class (pair-free mode)
+  // by gene: positions [0, cut) of `order` are the tensor cores' for this target
+  // (te_mma.cu); nullptr without that launch
+  const int32_t* cut;
   // pair-list mode (pairs != nullptr): item q is pairs[item_start[q] .. item_start[q+1])
   // of one target; output index = position in the list
   const int64_t* pairs;
@@ -759,6 +761,7 @@ __global__ void __launch_bounds__(1024, 1) te_pair_tile_kernel(TeParams P) {
       lo = (int64_t)chunk * P.W;
       hi = min((int64_t)(chunk + 1) * P.W, (int64_t)P.n);
       if (base + nm1 <= P.p0 || base >= P.p1) lo = hi;  // target outside the range
+      if (P.cut) lo = max(lo, (int64_t)P.cut[tgt]);
       // sources are sorted by bin count: skip a chunk this launch has no pair of
       if (P.overflow && lo < hi) {
         const int btq = P.npv[tgt];
@@ -914,74 +917,6 @@ __global__ void __launch_bounds__(1024, 1) te_pair_tile_kernel(TeParams P) {
   }
 }
 
-// Per-gene pre-pass: validation (every bin of gene g in [0, row_len) below
-// n_per_var[g], and 1 <= n_per_var[g] <= b_max; sets ws->bad_data otherwise).
-// One CTA per gene.
-__global__ void gene_prepass_kernel(const uint8_t* bins, int64_t ld, const int32_t* npv,
-                                    int b_max, int n, int64_t row_len, WsHeader* ws) {
-  const int g = blockIdx.x;
-  if (g >= n) return;
-  const int b = npv[g];
-  const uint8_t* row = bins + (int64_t)g * ld;
-  const int64_t nvec = row_len >> 4;
-  bool bad = b < 1 || b > b_max;
-  const uint4* rv = reinterpret_cast<const uint4*>(row);
-  for (int64_t v = threadIdx.x; v < nvec; v += blockDim.x) {
-    const uint4 q = __ldg(rv + v);
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-      for (int bb = 0; bb < 4; ++bb) bad |= ((w[k] >> (8 * bb)) & 0xffu) >= (uint32_t)b;
-  }
-  for (int64_t i = (nvec << 4) + threadIdx.x; i < row_len; i += blockDim.x) bad |= row[i] >= b;
-  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicExch(&ws->bad_data, 1);
-}
-
-// Source order for pair-free items: genes stably sorted by bin count, so a work
-// item's sources have similar b (its histogram slots are sized for them) and the
-// pairs that overflow shared memory form a suffix of every target's order. One CTA of 1024 threads;
-// deterministic (ballot + block scan, no atomics on the order).
-__device__ __forceinline__ int order_class(int b) {
-  return b < 0 ? 0 : (b > 255 ? 255 : b);  // out-of-range counts (rejected later) stay in bounds
-}
-
-__global__ void __launch_bounds__(1024) source_order_kernel(const int32_t* __restrict__ npv,
-                                                            int n, int32_t* __restrict__ order) {
-  constexpr int kClasses = 256;
-  __shared__ int present[kClasses];
-  __shared__ int wsum[32];
-  __shared__ int base_sh;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-  for (int c = tid; c < kClasses; c += blockDim.x) present[c] = 0;
-  if (tid == 0) base_sh = 0;
-  __syncthreads();
-  for (int g = tid; g < n; g += blockDim.x) present[order_class(npv[g])] = 1;
-  __syncthreads();
-  for (int c = 0; c < kClasses; ++c) {
-    if (!present[c]) continue;  // uniform: read after the barrier above
-    for (int start = 0; start < n; start += blockDim.x) {
-      const int g = start + tid;
-      const int flag = (g < n) && order_class(npv[g]) == c;
-      const unsigned m = __ballot_sync(0xffffffffu, flag);
-      const int pre = __popc(m & ((1u << lane) - 1u));
-      if (lane == 0) wsum[w] = __popc(m);
-      __syncthreads();
-      int wpre = 0, tot = 0;
-      for (int k = 0; k < nw; ++k) {
-        const int v = wsum[k];
-        wpre += k < w ? v : 0;
-        tot += v;
-      }
-      const int b0 = base_sh;
-      if (flag) order[b0 + wpre + pre] = g;
-      __syncthreads();
-      if (tid == 0) base_sh = b0 + tot;
-      __syncthreads();
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -1132,13 +1067,19 @@ extern "C" int tenex_te_launch_shape(int64_t row_len, int64_t lag, int b_max,
   return TENEX_OK;
 }
 
-extern "C" size_t tenex_te_workspace_bytes(int n_vars, int64_t row_len, int b_max) {
+extern "C" size_t tenex_te_pairs_workspace_bytes(int n_vars, int64_t row_len, int b_max) {
   if (n_vars < 1 || b_max < 1) return sizeof(WsHeader);
   size_t total = (size_t)ws_total(n_vars, b_max);
   DevAttr A;
   if (row_len > 1 && row_len < ((int64_t)1 << 31) && current_device_attr(&A) == TENEX_OK)
     total += (size_t)gmem_bytes(b_max, (int)row_len, b_max <= 16 ? 1 : 2, A);
   return total;
+}
+
+extern "C" size_t tenex_te_workspace_bytes(int n_vars, int64_t row_len, int b_max) {
+  const size_t base = tenex_te_pairs_workspace_bytes(n_vars, row_len, b_max);
+  if (n_vars < 2 || b_max < 1 || b_max > 255 || row_len < 2) return base;
+  return (size_t)round_up((int64_t)base, 256) + (size_t)te_mma_bytes(n_vars, row_len, b_max);
 }
 
 extern "C" int tenex_workspace_status(const void* workspace, void* stream) {
@@ -1156,6 +1097,8 @@ extern "C" int tenex_workspace_status(const void* workspace, void* stream) {
     return fail(TENEX_ERR_BADDATA,
                 "a bin value was >= its gene's n_per_var, or n_per_var was outside [1, b_max]; "
                 "no TE was computed");
+  if (h.bad_item == 2)
+    return fail(TENEX_ERR_TIMEOUT, "a tensor-core pipeline wait expired; results invalid");
   if (h.bad_item) return fail(TENEX_ERR_UNSUPPORTED,
                               "a work item's histogram did not fit shared memory");
   return TENEX_OK;
@@ -1274,7 +1217,7 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   // pairs whose histogram does not fit shared memory, and every pair of a target
   // beyond the marginal bound: global-memory overflow launch
   const bool overflow = needs_overflow(b_max, P.N, P.zbytes, P.mbmax, L.smem);
-  int64_t n_gslots = 0;
+  int64_t n_gslots = 0, ws_used = ws_total(n, b_max);
   if (overflow) {
     P.gslot_words = (int64_t)b_max * b_max * b_max;
     n_gslots = gmem_slot_count(b_max, A);
@@ -1296,21 +1239,44 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
     }
     P.gc2b = reinterpret_cast<uint32_t*>(g + slot_bytes + marg_bytes);
     P.gc2b_words = gc2b_words(b_max);
+    ws_used = round_up(need, 256);
   }
   P.overflow = overflow ? 1 : 0;
   int64_t grid = L.grid;
   if (grid > P.n_items) grid = P.n_items;
 
+  TeMma M{};
+  M.bins = bins;
+  M.ld = ld;
+  M.npv = npv;
+  M.n = n;
+  M.N = P.N;
+  M.inv_N = 1.0 / (double)P.N;
+  M.lag = P.lag;
+  M.b_max = b_max;
+  M.row_len = row_len;
+  M.p0 = P.p0;
+  M.p1 = P.p1;
+  M.t_first = P.t_first;
+  M.t_last = P.t_first + P.n_targets - 1;
+  M.ws = P.ws;
+  M.order = order;
+  M.out_mode = out_mode;
+  M.out = out;
+  M.out_ld = out_ld;
+  M.obs = obs;
+  M.sum = sum;
+  M.sumsq = sumsq;
+  M.cnt_ge = cnt;
+  M.counts_dbg = counts;
+  M.counts_stride = counts_stride;
+  // pairs of few cells go to the tensor cores where the workspace has room for their
+  // tables and bit planes (one sized by tenex_te_workspace_bytes has)
+  if (!pairs && te_mma_layout(&M, wsb + ws_used, (int64_t)ws_bytes - ws_used)) P.cut = M.cut;
   cudaError_t e = cudaMemsetAsync(workspace, 0, sizeof(WsHeader), stream);
   if (e != cudaSuccess) return check_cuda(e, "workspace reset");
-  gene_prepass_kernel<<<n, 256, 0, stream>>>(bins, ld, npv, b_max, n, row_len, P.ws);
-  st = check_launch("gene_prepass_kernel");
-  if (st) return st;
-  if (!pairs) {
-    source_order_kernel<<<1, 1024, 0, stream>>>(npv, n, order);
-    st = check_launch("source_order_kernel");
-    if (st) return st;
-  }
+  st = te_mma_launch(M, A, pairs != nullptr, stream);
+  if (st || (P.cut && te_mma_takes_all(M))) return st;
   e = cudaFuncSetAttribute(te_pair_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            L.smem);
   if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute");

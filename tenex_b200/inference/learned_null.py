@@ -408,7 +408,7 @@ def fallback_surrogates(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: in
     ssum = torch.zeros((n, n), dtype=torch.float64, device=dev)
     ssq = torch.zeros((n, n), dtype=torch.float64, device=dev)
     cnt = torch.zeros((n, n), dtype=torch.int32, device=dev)
-    ws = D.workspace(dev, n, db.row_len, b_max)
+    ws = D.workspace(dev, n, db.row_len, b_max, pair_list=True)
 
     def one(k):
         D.block_shuffle(db, perms[k], bl, out=shuf)
@@ -474,7 +474,7 @@ def fallback_surrogates_batched(db: D.DeviceBins, npv: torch.Tensor, b_max: int,
         items_big = torch.cat([(it_d[:-1][None, :] + (off * P)[:, None]).reshape(-1),
                                torch.tensor([kk * P], dtype=torch.int64, device=dev)])
         npv_big = npv.to(torch.int32).repeat(kk).contiguous()
-        ws = D.workspace(dev, kk * n, db.row_len, b_max)
+        ws = D.workspace(dev, kk * n, db.row_len, b_max, pair_list=True)
         te = torch.empty(kk * P, dtype=torch.float32, device=dev)
         native.call("tenex_te_pairs", big.ptr(), big.ld, npv_big.data_ptr(), int(b_max),
                     kk * n, big.row_len, lag, pairs_big.data_ptr(), kk * P, items_big.data_ptr(),

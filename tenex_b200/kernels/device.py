@@ -220,8 +220,18 @@ def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else int(t.data_ptr())
 
 
-def workspace(device, n: int, row_len: int, b_max: int) -> torch.Tensor:
-    nb = int(native.lib().tenex_te_workspace_bytes(int(n), int(row_len), int(b_max)))
+def workspace(device, n: int, row_len: int, b_max: int, pair_list: bool = False) -> torch.Tensor:
+    """Workspace of one TE call (pair_list: of a pair-list call, which needs less).
+    Where the device has no room for the tensor-core path's tables and bit planes,
+    the call gets the least it needs and runs without them."""
+    L = native.lib()
+    if not pair_list:
+        nb = int(L.tenex_te_workspace_bytes(int(n), int(row_len), int(b_max)))
+        try:
+            return torch.empty(nb, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            pass
+    nb = int(L.tenex_te_pairs_workspace_bytes(int(n), int(row_len), int(b_max)))
     return torch.empty(nb, dtype=torch.uint8, device=device)
 
 

@@ -47,7 +47,7 @@ def te_pair_list(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: int, pair
     pairs_d = torch.from_numpy(sp).to(dev)
     items_d = torch.from_numpy(items).to(dev)
     npv = npv.to(device=dev, dtype=torch.int32).contiguous()
-    ws = D.workspace(dev, db.n, db.row_len, b_max)
+    ws = D.workspace(dev, db.n, db.row_len, b_max, pair_list=True)
     s = native.stream_ptr()
     tmp = torch.empty(P, dtype=torch.float32, device=dev)
     native.call("tenex_te_pairs", db.ptr(), db.ld, npv.data_ptr(), int(b_max), db.n,

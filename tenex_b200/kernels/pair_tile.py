@@ -143,7 +143,7 @@ class PairTileKernel(TEKernel):
         tgt = ids // n_src
         pairs = torch.stack((tgt, n_tgt + ids - tgt * n_src), dim=1).contiguous()
         items = torch.from_numpy(item_table(tgt.cpu().numpy(), 128)).to(dev)
-        ws = D.workspace(dev, db.n, db.row_len, b_max)
+        ws = D.workspace(dev, db.n, db.row_len, b_max, pair_list=True)
         s = native.stream_ptr()
         native.call("tenex_te_pairs", db.ptr(), db.ld, npv.data_ptr(), b_max, db.n,
                     db.row_len, tau * db.K, pairs.data_ptr(), n_pairs_local, items.data_ptr(),

@@ -60,6 +60,7 @@ _SIGS = {
     "tenex_last_error": [ctypes.c_char_p, _S],
     "tenex_device_query": [_I, ctypes.POINTER(DevInfo)],
     "tenex_te_workspace_bytes": [_I, _L, _I],
+    "tenex_te_pairs_workspace_bytes": [_I, _L, _I],
     "tenex_te_launch_shape": [_L, _L, _I, _P, _P, _P, _P, _P],
     "tenex_workspace_status": [_P, _P],
     "tenex_te_pairfree": [_P, _L, _P, _I, _I, _L, _L, _L, _L, _P, _I, _L, _P, _S,
@@ -114,6 +115,7 @@ _SIGS = {
                            _P],
 }
 _RESTYPES = {"tenex_te_workspace_bytes": ctypes.c_size_t,
+             "tenex_te_pairs_workspace_bytes": ctypes.c_size_t,
              "tenex_b2_workspace_bytes": ctypes.c_size_t,
              "tenex_mlp_scratch_floats": ctypes.c_size_t,
              "tenex_eiid_workspace_bytes": ctypes.c_size_t}

@@ -1,0 +1,120 @@
+"""Tensor-core histograms (te_mma.cu) against the oracle and against the
+shared-memory kernel, which takes every pair when the workspace has no room for the
+tensor-core path's tables and bit planes.
+
+Counts are whole numbers and compared exactly. TE: both kernels evaluate the same
+float32 expression per cell and differ in the order of the sums; a term's rounding is
+at most 2^-23 of its count, so two sums of N counts differ by less than 1e-6 per
+sample."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from tenex_b200 import native
+from tenex_b200.kernels import device as D
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-6
+
+
+def _bins(seed, n, T, b_lo, b_hi, K=1, skew=False):
+    rng = np.random.default_rng(seed)
+    b = rng.integers(b_lo, b_hi + 1, n)
+    x = np.stack([rng.integers(0, v, T * K) for v in b])
+    if skew:  # rare bins: target states that never occur, empty (xt, y) columns
+        x = np.where(rng.random(x.shape) < 0.8, 0, x)
+    bins, npv, bmax = O.remap(x.astype(np.int32))
+    return bins.reshape(n, T, K), npv, bmax
+
+
+def _run(db, npv, bmax, lag, p0, cnt, dev, tensor_cores, matrix=False, counts=None):
+    """(TE, raw counts) of pair ids [p0, p0 + cnt) through the C ABI; tensor_cores =
+    False gives the call the workspace of the shared-memory kernel only."""
+    full = D.workspace(dev, db.n, db.row_len, bmax)
+    ws = full if tensor_cores else D.workspace(dev, db.n, db.row_len, bmax, pair_list=True)
+    out = torch.zeros((db.n, db.n) if matrix else cnt, dtype=torch.float32, device=dev)
+    s = native.stream_ptr()
+    if counts is None:
+        native.call("tenex_te_pairfree", db.ptr(), db.ld, npv.data_ptr(), bmax, db.n, db.row_len,
+                    lag, p0, cnt, out.data_ptr(),
+                    native.OUT_MATRIX if matrix else native.OUT_PAIRFREE, db.n if matrix else 0,
+                    ws.data_ptr(), ws.numel(), None, s)
+    else:
+        native.call("tenex_te_pairfree_counts", db.ptr(), db.ld, npv.data_ptr(), bmax, db.n,
+                    db.row_len, lag, p0, cnt, out.data_ptr(), counts.data_ptr(), bmax ** 3,
+                    ws.data_ptr(), ws.numel(), None, s)
+    native.call("tenex_workspace_status", ws.data_ptr(), s)
+    return out
+
+
+# (genes, samples, bins, lag): one gene pair; sample counts around the 64-sample MMA,
+# the 256-sample step and the ring of stages; lags past a word and past a step; bins
+# around the largest target (16), rows that fill a tile unevenly, wide sources
+SHAPES = [(2, 2, (1, 3), 1), (3, 65, (2, 4), 1), (9, 256, (2, 2), 1), (9, 257, (2, 5), 1),
+          (12, 320, (3, 7), 33), (40, 769, (2, 9), 1), (150, 511, (1, 2), 1),
+          (70, 1030, (2, 16), 3), (60, 1500, (13, 16), 1), (30, 2049, (2, 38), 300),
+          (25, 700, (5, 38), 1), (131, 1024, (4, 4), 1)]
+
+
+@pytest.mark.parametrize("n,T,b,lag", SHAPES)
+@pytest.mark.parametrize("skew", [False, True])
+def test_counts_and_te(cuda, n, T, b, lag, skew):
+    bins, npv, bmax = _bins(n * T + skew, n, T, *b, skew=skew)
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P = n * (n - 1)
+    ref = O.te_pairfree(bins, npv, tau=lag)
+    lo, hi = (P // 3, P - P // 5) if P > 6 else (0, P)   # a range that cuts targets
+    te = [_run(db, npv_t, bmax, lag, 0, P, cuda, tc).cpu().numpy() for tc in (True, False)]
+    assert np.max(np.abs(te[0] - ref)) <= TOL
+    assert np.max(np.abs(te[0] - te[1])) <= TOL
+    part = _run(db, npv_t, bmax, lag, lo, hi - lo, cuda, True).cpu().numpy()
+    # a pair's value does not depend on the range, so not on its tile
+    few = (bmax ** 3 <= 1200)
+    assert np.max(np.abs(part - te[0][lo:hi])) <= (0 if few else TOL)
+    m = _run(db, npv_t, bmax, lag, 0, P, cuda, True, matrix=True).cpu().numpy()
+    assert np.array_equal(m.T[~np.eye(n, dtype=bool)], te[0]) and not m.diagonal().any()
+    if P * bmax ** 3 <= 40_000_000:
+        c = [torch.full((P, bmax ** 3), -1, dtype=torch.int32, device=cuda) for _ in range(2)]
+        t = [_run(db, npv_t, bmax, lag, 0, P, cuda, tc, counts=k).cpu().numpy()
+             for tc, k in zip((True, False), c)]
+        assert torch.equal(c[0], c[1])
+        assert np.array_equal(t[0], te[0])
+
+
+def test_counts_exact_up_to_2_pow_24(cuda):
+    """float32 accumulators hold every count of the longest series the path takes:
+    constant genes give one cell of all N samples."""
+    T = (1 << 24) - 3
+    rng = np.random.default_rng(7)
+    x = np.zeros((4, T), np.uint8)
+    x[1] = rng.random(T) < 1e-6
+    x[2] = rng.random(T) < 0.5
+    x[1, 5], x[2, 9], x[3] = 1, 1, 1 - x[1]
+    npv = np.array([1, 2, 2, 2], np.int32)
+    db = D.pack_bins(x, cuda)
+    npv_t = torch.as_tensor(npv, device=cuda)
+    c = [torch.zeros((12, 8), dtype=torch.int32, device=cuda) for _ in range(2)]
+    te = [_run(db, npv_t, 2, 1, 0, 12, cuda, tc, counts=k) for tc, k in zip((True, False), c)]
+    assert torch.equal(c[0], c[1])
+    assert float((te[0] - te[1]).abs().max()) <= TOL
+
+
+def test_kernel_dimension_and_surrogate_statistics(cuda):
+    bins, npv, bmax = _bins(3, 45, 400, 2, 8, K=2)
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    te = D.te_pairfree(db, npv_t, bmax, 2, matrix=True)
+    ref = _run(db, npv_t, bmax, 4, 0, 45 * 44, cuda, False, matrix=True)
+    assert float((te - ref).abs().max()) <= TOL
+    obs = torch.full((45, 45), float(te.median()), device=cuda)
+    acc = [torch.zeros((45, 45), dtype=torch.float64, device=cuda) for _ in range(2)]
+    cnt = torch.zeros((45, 45), dtype=torch.int32, device=cuda)
+    for _ in range(2):
+        D.surrogate_accumulate(db, npv_t, bmax, 2, obs, acc[0], acc[1], cnt)
+    off = ~torch.eye(45, dtype=torch.bool, device=cuda)
+    assert torch.equal(acc[0], 2 * te.double())
+    assert torch.equal(acc[1], 2 * te.double() ** 2)
+    assert torch.equal(cnt[off], 2 * (te >= obs).int()[off])
+    assert not cnt[~off].any()
