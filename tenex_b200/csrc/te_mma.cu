@@ -6,11 +6,10 @@
 // So the histograms of all pairs are one matrix product: rows = (source, y), columns
 // = (target, occupied state (xt1, xt)), K = samples. It costs one multiply-add per
 // cell and sample where counting costs one shared-memory reduction per sample
-// (2.2e12 of them per second), so pairs of up to kMaxCells cells come here and the
+// (2.2e12 of them per second), so pairs of few cells come here (te_mma_layout) and the
 // others stay with te_pair.cu. Measured, all pairs, counting alone -> with this path:
-// 10,000 genes x 20,000 samples (b to 16, 5% to 38) 928 -> 705 ms, 2,000 x 5,000
-// (b to 16) 11.3 -> 8.6 ms, 3,281 x 458 (b to 7, every pair here) 7.1 -> 2.2 ms,
-// 301 x 101,003 (b to 12) 6.1 -> 3.4 ms.
+// 10,000 genes x 20,000 samples (b to 16, 5% to 38) 928 -> 662 ms, 2,000 x 5,000
+// (b to 16) 11.3 -> 7.8 ms, 3,281 x 458 (b to 7, every pair here) 7.1 -> 1.8 ms.
 //
 //   * plan (one CTA): sources sorted by bin count and targets by occupied states are
 //     cut into tiles of at most 128 rows and 240 columns, whole genes only, so a
@@ -28,10 +27,12 @@
 //     could not deliver.
 //   * epilogue: a TMEM lane is one (source, y); it walks the columns of each target by
 //     xt, so c2b is a sum of its own registers. The terms are te_pair.cu's, operation
-//     for operation; sums over xt1 are float32, over xt and y float64.
-//   * Bound: the producers. A 256-sample step of a 256 x 240 tile takes a CTA pair
-//     about 1,100 cycles with two pairs on the SMs' shared-memory and logic pipes; its
-//     MMAs alone take under 400 (measured with operands left as they were).
+//     for operation; a lane's sum over a target's (or half a target's) columns is
+//     float32, as long a chain as te_pair.cu's, those over y are float64.
+//   * Bound: the shared-memory pipe (about 520 cycles per SM for a 256-sample step of a
+//     256 x 240 tile: operands written, read by the MMAs, and the planes' loads; ncu: the
+//     load-store part of it 66% of the cycles, the tensor pipe 62%, the logic pipe 55%).
+//     The MMAs alone take under 390 (timed with operands left as they were).
 //   * Two CTAs share an SM (256 TMEM columns each): one's epilogue runs under the
 //     other's contraction. Work items go round the CTA pairs in an order that takes 16
 //     source tiles at a time across all target tiles, so the planes in use stay in L2.
@@ -48,7 +49,6 @@
 namespace tenex {
 namespace {
 
-constexpr int kMaxCells = 1200;   // occupied target states x source bins of a pair
 constexpr int kMaxTgtBins = 16;   // target bins (at most 16 columns share an xt)
 constexpr int kMaxCols = 240;     // columns of a tile
 constexpr int kRows = 128;        // rows of a tile (TMEM lanes) per CTA of a pair
@@ -64,7 +64,7 @@ constexpr int kTmemCols = 256;
 // Partial sums of a tile: one float64 row of kRows per target, two for targets of
 // kSplitCols columns or more (those of kSplitBins bins or more, which have at least
 // kSplitBins - 1 columns, are summed by two warps per lane quarter).
-constexpr int kSlots = 60, kSplitCols = 7, kSplitBins = 8;
+constexpr int kSlots = 56, kSplitCols = 7, kSplitBins = 8;
 constexpr int kBlkCache = 128;    // item blocks whose starts sit in shared memory
 static_assert(kSlots * kRows * 8 <= kStages * kStageBytes, "partial sums fit the stages");
 
@@ -299,12 +299,12 @@ __global__ void __launch_bounds__(1024) plan_kernel(TeMma M) {
   }, tid);
   const int n_stiles = S.n_tiles;
   // how many source positions each target takes: those with bins x columns within
-  // kMaxCells (S.base still holds the sources' class starts)
+  // max_cells (S.base still holds the sources' class starts)
   for (int g = tid; g < n; g += 1024) {
     int nc = M.ncols[g], cut = 0;
     if (M.rowoff[g] < 0) nc = 0;
     if (nc > 0) {
-      const int c = kMaxCells / nc;
+      const int c = M.max_cells / nc;
       cut = min(c >= 255 ? n : S.base[c + 1], n_src);
       if (cut == 0) nc = 0;
     }
@@ -477,17 +477,23 @@ __device__ __forceinline__ uint4 expand_col(uint32_t m) {
   return make_uint4((m << 2) & 0x44444444u, m & 0x22222222u, d & 0x11111111u, d & 0x22222222u);
 }
 
-// Sum over the L states xt1 of one xt (this lane's source bin y) of te_pair.cu's
-// terms: c log2(c (1 / c2b) (c1 / c2a)), exactly 0 where c c1 == c2a c2b. An empty
-// cell has a ratio of 0 (or, in an empty column, a NaN: fmaxf returns the other
-// operand), so its term is 0 times a finite logarithm.
+// acc plus the sum over the L states xt1 of one xt (this lane's source bin y) of
+// te_pair.cu's terms: c log2(c (1 / c2b) (c1 / c2a)), exactly 0 where c c1 == c2a c2b.
+// The reciprocal is the hardware's approximation and one Newton-Raphson step with fused
+// multiply-adds (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990): equal to __frcp_rn for every whole number up to 2^24
+// (checked one by one), a quarter of its instructions. An empty cell has a ratio of 0,
+// so its term is 0 times a finite logarithm.
 template <int L, int R>
-__device__ __forceinline__ float group_terms(const uint32_t (&r)[R], const float2* q, float c1) {
-  float b = 0.f;
+__device__ __forceinline__ float group_terms(float acc, const uint32_t (&r)[R], const float2* q,
+                                             float c1) {
+  float b = __uint_as_float(r[0]);
 #pragma unroll
-  for (int u = 0; u < L; ++u) b += __uint_as_float(r[u]);
-  const float inv = __frcp_rn(fmaxf(b, 1.f));
-  float acc = 0.f;
+  for (int u = 1; u < L; ++u) b += __uint_as_float(r[u]);
+  const float d = fmaxf(b, 1.f);
+  float inv;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(d));
+  inv = fmaf(inv, fmaf(-d, inv, 1.f), inv);
 #pragma unroll
   for (int u = 0; u < L; ++u) {
     const float c = __uint_as_float(r[u]);
@@ -495,38 +501,38 @@ __device__ __forceinline__ float group_terms(const uint32_t (&r)[R], const float
     const float x = fmaxf(c * inv * qu.x, 1e-30f);
     float t;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
-    const float with = fmaf(c, t, acc);
-    acc = c * c1 == qu.y * b ? acc : with;
+    if (c * c1 != qu.y * b) acc = fmaf(c, t, acc);
   }
   return acc;
 }
 
-__device__ __forceinline__ float group_sum(uint32_t taddr, int len, const float2* q, float c1) {
+__device__ __forceinline__ float group_sum(float acc, uint32_t taddr, int len, const float2* q,
+                                           float c1) {
   if (len <= 8) {
     uint32_t r[8];
     tmem_ld(taddr, r);
     switch (len) {
-      case 1: return group_terms<1>(r, q, c1);
-      case 2: return group_terms<2>(r, q, c1);
-      case 3: return group_terms<3>(r, q, c1);
-      case 4: return group_terms<4>(r, q, c1);
-      case 5: return group_terms<5>(r, q, c1);
-      case 6: return group_terms<6>(r, q, c1);
-      case 7: return group_terms<7>(r, q, c1);
-      default: return group_terms<8>(r, q, c1);
+      case 1: return group_terms<1>(acc, r, q, c1);
+      case 2: return group_terms<2>(acc, r, q, c1);
+      case 3: return group_terms<3>(acc, r, q, c1);
+      case 4: return group_terms<4>(acc, r, q, c1);
+      case 5: return group_terms<5>(acc, r, q, c1);
+      case 6: return group_terms<6>(acc, r, q, c1);
+      case 7: return group_terms<7>(acc, r, q, c1);
+      default: return group_terms<8>(acc, r, q, c1);
     }
   }
   uint32_t r[16];
   tmem_ld(taddr, r);
   switch (len) {
-    case 9: return group_terms<9>(r, q, c1);
-    case 10: return group_terms<10>(r, q, c1);
-    case 11: return group_terms<11>(r, q, c1);
-    case 12: return group_terms<12>(r, q, c1);
-    case 13: return group_terms<13>(r, q, c1);
-    case 14: return group_terms<14>(r, q, c1);
-    case 15: return group_terms<15>(r, q, c1);
-    default: return group_terms<16>(r, q, c1);
+    case 9: return group_terms<9>(acc, r, q, c1);
+    case 10: return group_terms<10>(acc, r, q, c1);
+    case 11: return group_terms<11>(acc, r, q, c1);
+    case 12: return group_terms<12>(acc, r, q, c1);
+    case 13: return group_terms<13>(acc, r, q, c1);
+    case 14: return group_terms<14>(acc, r, q, c1);
+    case 15: return group_terms<15>(acc, r, q, c1);
+    default: return group_terms<16>(acc, r, q, c1);
   }
 }
 
@@ -537,9 +543,11 @@ struct Tables {
   int wide0;             // first target of kSplitCols columns or more (targets ascend)
   float2 q[kMaxCols];    // M.colq
   int2 row[kMaxCols / 2];     // M.colrow of the columns this CTA expands
-  uint32_t grp[kSlots * 16];  // M.grp
+  float c1[kSlots * 16];      // M.grp
+  uint8_t len[kSlots * 16];
   int4 tgt[kSlots];      // M.tgt
-  int2 src[kRows + 1];   // gene, first row in the tile; then the number of rows
+  int src[kRows];             // genes of the sources
+  uint8_t at[kRows + 1];      // their first rows in the tile; then the number of rows
 };
 
 struct Shared {
@@ -594,7 +602,7 @@ __device__ void next_item(const TeMma& M, Shared& S, Tables& T, uint32_t* q_io, 
   if (lane == 0) {
     T.st = st;
     T.tt = tt;
-    T.src[st.y] = make_int2(0, st.w);
+    T.at[st.y] = (uint8_t)st.w;
   }
   for (int c = lane; c < tt.w; c += 32) T.q[c] = M.colq[tt.z + c];
   const int n_half = (tt.w + 15) / 16 * 8, c0 = (int)rank * n_half;
@@ -607,10 +615,15 @@ __device__ void next_item(const TeMma& M, Shared& S, Tables& T, uint32_t* q_io, 
   }
   narrow = __reduce_add_sync(0xffffffffu, narrow);
   if (lane == 0) T.wide0 = narrow;
-  for (int k = lane; k < tt.y * 16; k += 32) T.grp[k] = M.grp[(int64_t)tt.x * 16 + k];
+  for (int k = lane; k < tt.y * 16; k += 32) {
+    const uint32_t g = M.grp[(int64_t)tt.x * 16 + k];
+    T.c1[k] = (float)(g & 0xffffffu);
+    T.len[k] = (uint8_t)(g >> 24);
+  }
   for (int s = lane; s < st.y; s += 32) {
     const int2 v = M.src[st.x + s];
-    T.src[s] = make_int2(v.x, v.y - st.z);
+    T.src[s] = v.x;
+    T.at[s] = (uint8_t)(v.y - st.z);
   }
 }
 
@@ -635,12 +648,12 @@ __device__ __forceinline__ void put_pair(const TeMma& M, int src, int tgt, doubl
 // Raw counts of this lane's (source, y) for target tt (parity checks only).
 __device__ void put_counts(const TeMma& M, const Tables& T, int tt, int row, uint32_t lane_base) {
   int s = 0;
-  while (s < T.st.y && T.src[s + 1].y <= row) ++s;
+  while (s < T.st.y && T.at[s + 1] <= row) ++s;
   const bool mine = s < T.st.y;
   const int4 t = T.tgt[tt];
-  const int src = mine ? T.src[s].x : 0, tgt = t.x, bt = t.y;
+  const int src = mine ? T.src[s] : 0, tgt = t.x, bt = t.y;
   const int64_t p = (int64_t)tgt * (M.n - 1) + (src < tgt ? src : src - 1);
-  const int bs = mine ? T.src[s + 1].y - T.src[s].y : 1, y = mine ? row - T.src[s].y : 0;
+  const int bs = mine ? T.at[s + 1] - T.at[s] : 1, y = mine ? row - T.at[s] : 0;
   const bool put = mine && src != tgt && p >= M.p0 && p < M.p1;
   int32_t* cd = M.counts_dbg + (put ? (p - M.p0) * M.counts_stride : 0);
   if (put)
@@ -656,8 +669,12 @@ __device__ void put_counts(const TeMma& M, const Tables& T, int tt, int row, uin
 
 // Two CTAs (a pair of SMs) share an item: 256 rows, each CTA's own 128 in its TMEM;
 // each expands half of the columns and the even one issues for both
-// (cta_group::2), so a column is expanded once per 256 rows. 10,000 x 20,000: 245 ms,
-// against 315 ms with one CTA per 128-row tile.
+// (cta_group::2), so a column is expanded once per 256 rows. 10,000 x 20,000: 203 ms
+// (245 before the producers were split in two groups, the odd CTA's arrivals lost their
+// cluster-wide release and the epilogue its slow reciprocals and float64 sums), against
+// 315 ms with one CTA per 128-row tile. Row operands in TMEM instead of shared memory
+// (192 columns, three stages): 407 ms at a limit of 1,600 cells against 311 here; the
+// ring is then too short for its round trip of about 1,200 cycles.
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_kernel(TeMma M) {
   if (*(volatile int*)&M.ws->bad_data != 0) return;
   const int n_items = M.ws->mma_items, n_blk = M.ws->mma_blocks, n_stiles = M.ws->mma_stiles;
@@ -673,7 +690,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
       // the issuing CTA's: one more arrival for the other CTA's half
-      mbar_init(&S.full[s], kProducers / 32 + (rank == 0 ? 1 : 0));
+      mbar_init(&S.full[s], 2 * kProducers / 64);
       mbar_init(&S.empty[s], 1);
     }
     mbar_init(&S.acc, 1);
@@ -709,71 +726,81 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
     const int n_tgts = T.tt.y, n_cols = T.tt.w, n_rows = T.st.w, wide0 = T.wide0;
     const int n_mma = (n_cols + 15) & ~15;  // columns of the MMAs, half from each CTA
     if (tid < kProducers) {
-      // ---- producers: lane pairs take half a step each of one row of this CTA's and
-      // of one column of its half. A store phase (eight lanes) covers four rows and both
-      // halves: all 32 banks once. Words for the next step are loaded before this one's
+      // ---- producers: warps 0-3 fill the even steps, warps 4-7 the odd ones. A lane
+      // pair takes half a step each of rows r and r + 64 of this CTA's and of columns r
+      // and r + 64 of its half; a store phase (eight lanes) covers four rows and both
+      // halves: all 32 banks once. Words of the next step are loaded before this one's
       // are expanded.
-      const int r = tid >> 1, half = tid & 1;
-      const bool a_on = r < n_rows;
-      const bool b_on = r < (n_mma >> 1) && (int)rank * (n_mma >> 1) + r < n_cols;
-      const int2 cr = b_on ? T.row[r] : make_int2(0, 0);
+      const int r = (tid & 127) >> 1, half = tid & 1, hc = n_mma >> 1;
+      const int nb = min(hc, n_cols - (int)rank * hc);  // columns to expand here
+      const bool a0_on = r < n_rows, a1_on = r + 64 < n_rows, b0_on = r < nb, b1_on = r + 64 < nb;
+      const int2 c0 = b0_on ? T.row[r] : make_int2(0, 0);
+      const int2 c1 = b1_on ? T.row[r + 64] : make_int2(0, 0);
+      const uint32_t oa = (uint32_t)(T.st.z + (a0_on ? r : 0)) * 2 + half;
+      const uint32_t oa1 = oa + (a1_on ? 128 : 0);
+      const uint32_t of0 = (uint32_t)c0.x * 2 + half, oq0 = (uint32_t)c0.y * 2 + half;
+      const uint32_t of1 = (uint32_t)c1.x * 2 + half, oq1 = (uint32_t)c1.y * 2 + half;
+      const uint32_t sw = (uint32_t)((r & 7) ^ (half << 2)) << 4;  // all four rows'
       const int64_t stride = M.cap_rows * 2;  // 256 samples on
-      const uint4* pa = reinterpret_cast<const uint4*>(M.P) + (a_on ? T.st.z + r : 0) * 2 + half;
-      const uint4* pf = reinterpret_cast<const uint4*>(M.F) + cr.x * 2 + half;
-      const uint4* pq = reinterpret_cast<const uint4*>(M.P) + cr.y * 2 + half;
-      const uint32_t sw = (uint32_t)((r & 7) ^ (half << 2)) << 4;  // both operands' rows
       unsigned char* const op = stages + r * 128;
-      uint4 va = __ldg(pa), vf = __ldg(pf), vq = __ldg(pq);
-      uint32_t s = stage, ph = parity ^ 1;  // `empty` starts as if just released
-      for (int k = 0; k < n_steps; ++k) {
-        const uint32_t a[4] = {va.x, va.y, va.z, va.w};
-        const uint32_t b[4] = {vf.x & vq.x, vf.y & vq.y, vf.z & vq.z, vf.w & vq.w};
-        if (k + 1 < n_steps) {
-          pa += stride;
-          pf += stride;
-          pq += stride;
-          va = __ldg(pa);
-          vf = __ldg(pf);
-          vq = __ldg(pq);
+      int k = warp >> 2;
+      uint32_t s = stage + k, ph = parity ^ 1;  // `empty` starts as if just released
+      if (s >= kStages) {
+        s -= kStages;
+        ph ^= 1;
+      }
+      const uint4* Pk = reinterpret_cast<const uint4*>(M.P) + k * stride;
+      const uint4* Fk = reinterpret_cast<const uint4*>(M.F) + k * stride;
+      uint4 va0, va1, vf0, vq0, vf1, vq1;
+      if (k < n_steps) {
+        va0 = __ldg(Pk + oa);
+        va1 = __ldg(Pk + oa1);
+        vf0 = __ldg(Fk + of0);
+        vq0 = __ldg(Pk + oq0);
+        vf1 = __ldg(Fk + of1);
+        vq1 = __ldg(Pk + oq1);
+      }
+      for (; k < n_steps; k += 2) {
+        const uint32_t a0[4] = {va0.x, va0.y, va0.z, va0.w};
+        const uint32_t a1[4] = {va1.x, va1.y, va1.z, va1.w};
+        const uint32_t b0[4] = {vf0.x & vq0.x, vf0.y & vq0.y, vf0.z & vq0.z, vf0.w & vq0.w};
+        const uint32_t b1[4] = {vf1.x & vq1.x, vf1.y & vq1.y, vf1.z & vq1.z, vf1.w & vq1.w};
+        if (k + 2 < n_steps) {
+          Pk += 2 * stride;
+          Fk += 2 * stride;
+          va0 = __ldg(Pk + oa);
+          va1 = __ldg(Pk + oa1);
+          vf0 = __ldg(Fk + of0);
+          vq0 = __ldg(Pk + oq0);
+          vf1 = __ldg(Fk + of1);
+          vq1 = __ldg(Pk + oq1);
         }
         if (!mbar_wait(&S.empty[s], ph)) {
           *(volatile int*)&S.abort = 1;
           break;
         }
         unsigned char* const row = op + s * kStageBytes;
-        if (a_on) put_half<true>(row, sw, a);
-        if (b_on) put_half<false>(row + kABytes, sw, b);
+        if (a0_on) put_half<true>(row, sw, a0);
+        if (b0_on) put_half<false>(row + kABytes, sw, b0);
+        if (a1_on) put_half<true>(row + 64 * 128, sw, a1);
+        if (b1_on) put_half<false>(row + kABytes + 64 * 128, sw, b1);
         fence_proxy_async_smem();
         __syncwarp();
-        if (elected) mbar_arrive(&S.full[s]);
-        if (++s == kStages) {
-          s = 0;
-          ph ^= 1;
-        }
-      }
-    } else if (rank == 1) {
-      // ---- tells the issuing CTA of this one's stages (a cluster-wide release by
-      // each producer warp would wait for its loads of the next step) ---------------
-      uint32_t s = stage, ph = parity;
-      for (int k = 0; k < n_steps; ++k) {
-        if (!mbar_wait(&S.full[s], ph)) {
-          *(volatile int*)&S.abort = 1;
-          break;
-        }
         if (elected) mbar_arrive_cluster(&S.full[s], 0);
-        if (++s == kStages) {
-          s = 0;
+        s += 2;
+        if (s >= kStages) {
+          s -= kStages;
           ph ^= 1;
         }
       }
-    } else {
+    } else if (rank == 0) {
       // ---- MMA issue, for both CTAs. The whole warp runs the loop, so that stage
       // numbers and descriptors stay in uniform registers; one lane issues -----------
       const uint32_t idesc = idesc_mxf4(2 * kRows, n_mma);
       const uint32_t last = (uint32_t)(((M.N & 255) + 63) >> 6);  // MMAs of a short last step
       uint32_t s = stage, ph = parity;
       for (int k = 0; k < n_steps; ++k) {
-        if (!mbar_wait_cluster(&S.full[s], ph)) {
+        if (!mbar_wait(&S.full[s], ph)) {
           *(volatile int*)&S.abort = 1;
           break;
         }
@@ -830,17 +857,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
           }
           if (j1 > 0) {
             int at = c0;
-            for (int j = 0; j < j0; ++j) at += T.grp[tt * 16 + j] >> 24;
-            double sum = 0.0;
+            for (int j = 0; j < j0; ++j) at += T.len[tt * 16 + j];
+            float sum = 0.f;
             for (int j = j0; j < j1; ++j) {
-              const uint32_t g = T.grp[tt * 16 + j];
-              const int len = g >> 24;
+              const int len = T.len[tt * 16 + j];
               if (len > 0)
-                sum += (double)group_sum(lane_base + (uint32_t)at, len, T.q + at,
-                                         (float)(g & 0xffffffu));
+                sum = group_sum(sum, lane_base + (uint32_t)at, len, T.q + at, T.c1[tt * 16 + j]);
               at += len;
             }
-            part[(slot + (bt >= kSplitBins ? half : 0)) * kRows + row] = sum;
+            part[(slot + (bt >= kSplitBins ? half : 0)) * kRows + row] = (double)sum;
           }
           if (M.counts_dbg != nullptr && half == 0) put_counts(M, T, tt, row, lane_base);
         }
@@ -857,12 +882,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
       if (T.st.x + s >= t.w) continue;  // te_pair.cu's pair
       const double* a = part + (tt < wide0 ? tt : 2 * tt - wide0) * kRows;
       double tot = 0.0;
-      const int y1 = T.src[s + 1].y;
+      const int y1 = T.at[s + 1];
       if (t.y >= kSplitBins)
-        for (int y = T.src[s].y; y < y1; ++y) tot += a[y] + a[y + kRows];
+        for (int y = T.at[s]; y < y1; ++y) tot += a[y] + a[y + kRows];
       else
-        for (int y = T.src[s].y; y < y1; ++y) tot += a[y];
-      put_pair(M, T.src[s].x, t.x, tot);
+        for (int y = T.at[s]; y < y1; ++y) tot += a[y];
+      put_pair(M, T.src[s], t.x, tot);
     }
     __syncthreads();
   }
@@ -934,6 +959,14 @@ bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
   M->grp = reinterpret_cast<uint32_t*>(take((int64_t)n * 64));
   M->colq = reinterpret_cast<float2*>(take(cols * 16));
   M->colrow = reinterpret_cast<int2*>(M->colq + cols);
+  // A pair's cells (occupied target states x source bins) up to which the tensor cores
+  // are the faster: their time goes with cells x samples, the counting kernel's with
+  // samples plus, per cell, its own entropy pass. Measured, ms of both kernels at a limit
+  // of 1,000 / 1,200 / 1,600 / 2,100 / 2,600 cells: 10,000 genes x 20,000 samples 665 /
+  // 662 / 671 / 694 / 725; 2,000 x 5,000 8.03 / 7.83 / 7.83 / 7.91 / 8.18; 2,000 x 600
+  // (b to 16) 4.82 / 4.66 / 4.19 / 3.93 / 3.76.
+  const double N = M->N;
+  M->max_cells = N <= 2078.0 ? 4096 : (int)(1200.0 * N / (N - 1470.0));
   M->cap_rows = std::min<int64_t>(rows, (int64_t)1 << 29);
   M->P = reinterpret_cast<uint32_t*>(at);
   M->F = M->P + M->cap_rows * M->words;
@@ -942,7 +975,7 @@ bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
 
 bool te_mma_takes_all(const TeMma& M) {
   const int64_t b = M.b_max;
-  return b * b <= kMaxCols && b * b * b <= kMaxCells && (int64_t)M.n * b <= M.cap_rows;
+  return b * b <= kMaxCols && b * b * b <= M.max_cells && (int64_t)M.n * b <= M.cap_rows;
 }
 
 int te_mma_launch(const TeMma& M, const DevAttr& A, bool pair_list, cudaStream_t stream) {

@@ -25,6 +25,7 @@ struct TeMma {
   int32_t* order;    // (n,) genes stably sorted by bin count (sources)
   // the rest only when cap_rows > 0
   int64_t cap_rows;  // bit-plane rows there is room for
+  int max_cells;     // most cells of a pair of the tensor cores (a rule on N)
   int words;         // 32-bit words of a plane row (a multiple of 8)
   int32_t* rowoff;   // (n,) by gene: first plane row, -1 without planes
   int32_t* ncols;    // (n,) by gene: occupied target states, 0 = not a tensor-core target
@@ -36,7 +37,7 @@ struct TeMma {
   int4* stile;       // (n,) source tiles: first position, sources, first row, rows
   int4* ttile;       // (n,) target tiles: first position, targets, first column, columns
   int32_t* nst;      // (n,) source tiles a target tile runs against
-  int32_t* blk;      // (n / 8 + 2,) first work item of each block of source tiles
+  int32_t* blk;      // (n / 16 + 2,) first work item of each block of source tiles
   int32_t* c2a;      // (n, 256) by gene: counts of the target states
   uint32_t* grp;     // (n, 16) by position: c1 | columns << 24 of x_t = j
   float2* colq;      // per column: c1 / c2a, c2a

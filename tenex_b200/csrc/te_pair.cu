@@ -1161,8 +1161,16 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   P.p0 = p0;
   P.p1 = p0 + n_pairs;
   // 512 sources per item: fewer target stagings than 128 (3% faster at 10,000
-  // genes), and a chunk of 512 source rows still fits L2 beside the others
+  // genes), and a chunk of 512 source rows still fits L2 beside the others. Fewer where
+  // there are too few targets for 16 items per CTA (few genes, a short pair range): the
+  // items are uneven, and one round of them leaves most SMs idle at its end
+  // (301 genes x 101,003 samples: 1.88 -> 0.64 ms for the pairs counted here).
   P.W = (cfg && cfg->src_chunk) ? cfg->src_chunk : 512;
+  if (!pairs && !(cfg && cfg->src_chunk)) {
+    const int64_t targets = (p0 + n_pairs - 1) / (n - 1) - p0 / (n - 1) + 1;
+    const int64_t chunks = std::min<int64_t>((n + 31) / 32, 32 * A.sm_count / targets);
+    if (chunks > 1) P.W = (int)std::min<int64_t>(P.W, (n + chunks - 1) / chunks);
+  }
   if (P.W < 1) return fail(TENEX_ERR_BADARG, "src_chunk must be >= 1");
   if (pairs) {
     P.pairs = pairs;

@@ -23,11 +23,12 @@ from tenex_b200.kernels import device as D
 # a whole SM's shared memory)
 TUNE_SPACE = [(0, 0, 512), (1024, 1, 512), (512, 2, 512), (512, 2, 256), (1024, 1, 256),
               (256, 4, 128), (256, 4, 256), (512, 2, 128), (1024, 1, 128), (256, 2, 64)]
-# Without autotuning the library picks the shape; 512 sources per item. Measured
+# Without autotuning the library picks the shape; 512 sources per item, fewer for few
+# genes. Measured
 # (ms per all-pairs launch): 10,000 x 20,000 (b_max 38) 989 vs 1097 for the old
 # 2 x 512 / 128 default; 5,000 x 10,000 (b_max 32) 256.0 vs 258.8; 2,000 x 5,000
 # (b_max 16) 11.37 vs 11.78 (11.14 for the best tuned shape).
-DEFAULT_CFG = dict(threads=0, ctas_per_sm=0, src_chunk=512)
+DEFAULT_CFG = dict(threads=0, ctas_per_sm=0, src_chunk=0)
 _tune_cache: dict[tuple, dict] = {}
 
 
