@@ -35,7 +35,7 @@ def binarize(arr, method: str = "nonzero", device=None, q: float = 0.5, **_unuse
     dev = torch.device(device) if device is not None else torch.device("cuda", 0)
     x = torch.as_tensor(np.ascontiguousarray(arr, dtype=np.float32)) if not isinstance(
         arr, torch.Tensor) else arr.to(torch.float32)
-    x = x.to(dev).contiguous()
+    x = (D.to_device(x, dev) if x.device.type == "cpu" else x.to(dev)).contiguous()
     n, T = (int(s) for s in x.shape)
     db = D.empty_bins(n, T, 1, dev)
     npv = torch.empty(n, dtype=torch.int32, device=dev)

@@ -32,6 +32,40 @@ def item_table(tgt_sorted: np.ndarray, run: int = 128) -> np.ndarray:
     return np.concatenate([items, [P]]).astype(np.int64)
 
 
+def te_source_rows(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: int,
+                   sources: np.ndarray, cfg=None, run: int = 128,
+                   check_data: bool = True) -> torch.Tensor:
+    """(n, n) float32 device matrix with [src, tgt] = TE(src -> tgt) for the distinct
+    gene indices `sources` and every target, 0 elsewhere and on the diagonal. The
+    pair list (target-major, the sources in the given order, a source against itself
+    included and dropped from the result) is a regular grid, so it and its items are
+    made on the device: 150 sources x 2,003 targets host to host 23 -> 3.5 ms."""
+    dev = db.data.device
+    n, m = db.n, len(sources)
+    out = torch.zeros((n, n), dtype=torch.float32, device=dev)
+    if m == 0:
+        return out
+    src = torch.as_tensor(np.ascontiguousarray(sources, dtype=np.int64)).to(dev)
+    pairs = torch.empty((n, m, 2), dtype=torch.int64, device=dev)
+    pairs[:, :, 0] = torch.arange(n, device=dev)[:, None]
+    pairs[:, :, 1] = src[None, :]
+    starts = torch.arange(0, m, run, device=dev)
+    items = torch.full((n * len(starts) + 1,), n * m, dtype=torch.int64, device=dev)
+    items[:-1].view(n, -1).copy_(torch.arange(0, n * m, m, device=dev)[:, None] + starts)
+    npv = npv.to(device=dev, dtype=torch.int32).contiguous()
+    ws = D.workspace(dev, n, db.row_len, b_max, pair_list=True)
+    s = native.stream_ptr()
+    te = torch.empty((n, m), dtype=torch.float32, device=dev)
+    native.call("tenex_te_pairs", db.ptr(), db.ld, npv.data_ptr(), int(b_max), n, db.row_len,
+                tau * db.K, pairs.data_ptr(), n * m, items.data_ptr(), items.numel() - 1,
+                te.data_ptr(), ws.data_ptr(), ws.numel(), D._cfg(cfg), s)
+    if check_data:
+        native.call("tenex_workspace_status", ws.data_ptr(), s)
+    out[src] = te.t()
+    out[src, src] = 0.0
+    return out
+
+
 def te_pair_list(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: int, pairs: np.ndarray,
                  cfg=None, run: int = 128, check_data: bool = True) -> torch.Tensor:
     """float32 TE per pair (device tensor), pairs (P, 2) int = [target, source]."""

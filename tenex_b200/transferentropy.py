@@ -152,22 +152,19 @@ class TransferEntropyEngine:
         key = (n_vars, None if self._sources is None else tuple(self._sources))
         if key in self._pairs_cache:
             return self._pairs_cache[key]
+        inds = self._source_indices()
+        tgt = np.repeat(np.arange(n_vars, dtype=np.int64), len(inds))
+        src = np.tile(inds, n_vars)
+        pairs = np.stack((tgt, src), axis=1)[tgt != src]
+        self._pairs_cache[key] = pairs
+        return pairs
+
+    def _source_indices(self) -> np.ndarray:
+        """Positions of the source names, in the order of _build_pairs."""
         _, inds, _ = np.intersect1d(self._variable_names, self._sources, return_indices=True)
         if len(inds) == 0:
             raise ValueError("No source names found in variable_names.")
-        srcs = inds.astype(np.int64)
-        blocks = []
-        for t in range(n_vars):
-            s_valid = srcs[srcs != t]
-            if len(s_valid):
-                b = np.empty((len(s_valid), 2), np.int64)
-                b[:, 0] = t
-                b[:, 1] = s_valid
-                blocks.append(b)
-        pairs = np.concatenate(blocks) if blocks else np.empty((0, 2), np.int64)
-        pairs = pairs[np.argsort(pairs[:, 0], kind="stable")]
-        self._pairs_cache[key] = pairs
-        return pairs
+        return inds.astype(np.int64)
 
     @staticmethod
     def _select_kernel(kernel_name, b_max, on_cuda, smem_optin, smem_bytes, n_per_var,
@@ -279,20 +276,20 @@ class TransferEntropyEngine:
         mark(5)
         if source_filter:
             info.update(mode="pair", pair_free=False)
-            pairs = self._build_pairs(n_vars)
             if len(device_ids) > 1:
+                pairs = self._build_pairs(n_vars)
                 te_h = kobj.compute_multi_gpu(self._host_bins(work), pairs, b_max_w,
                                               npv_w.cpu(), tau, batch_size, device_ids)
                 mark(6)
+                rm = np.zeros((n_vars, n_vars), dtype=np.float32)
+                rm[pairs[:, 0], pairs[:, 1]] = te_h
+                self._result_matrix = rm.T.copy()
             else:
-                from tenex_b200.kernels.pair_list import te_pair_list
-                te = te_pair_list(work, npv_w, b_max_w, tau, pairs,
-                                  cfg=getattr(kobj, "cfg", None))
+                from tenex_b200.kernels.pair_list import te_source_rows
+                m = te_source_rows(work, npv_w, b_max_w, tau, self._source_indices(),
+                                   cfg=getattr(kobj, "cfg", None))
                 mark(6)
-                te_h = D.to_host(te)
-            rm = np.zeros((n_vars, n_vars), dtype=np.float32)
-            rm[pairs[:, 0], pairs[:, 1]] = te_h
-            self._result_matrix = rm.T.copy()
+                self._result_matrix = D.to_host(m)
         else:
             info.update(mode="pairfree", pair_free=True)
             if len(device_ids) > 1:
