@@ -187,54 +187,71 @@ __device__ void stable_order(PlanShared& S, int n, Key key, int32_t* order, int 
 // emit_tiles), those that span classes one by one.
 __device__ void pack_tiles(PlanShared& S, int c_lo, int c_hi, int room, int most, int dbl,
                            int limit, int tid) {
-  if (tid == 0) {
-    S.n_seg = S.n_open = 0;
-    int tile = 0, k = 0, used = 0, weight = 0, pos0 = 0;
-    for (int ci = 0; ci < S.n_cls; ++ci) {
-      const int c = S.cls[ci];
-      if (c < c_lo || c > c_hi) continue;
-      int pos = S.base[c];
-      int m = min(S.cnt[c], limit - pos);
-      if (m <= 0) break;
-      const int wt = c >= dbl ? 2 : 1;
-      const int per = min(room / c, most / wt);
-      if (k > 0) {
-        const int r = min(m, min((room - used) / c, (most - weight) / wt));
-        k += r;
-        used += r * c;
-        weight += r * wt;
-        pos += r;
-        m -= r;
-        if (m > 0) {
-          S.open_tile[S.n_open] = tile++;
-          S.open_pos[S.n_open] = pos0;
-          S.open_n[S.n_open++] = k;
-          k = 0;
-        }
+  // a serial chain over the classes: one warp, 32 classes at a time in its lanes, all
+  // lanes following the chain, quotients of numbers up to `room` by a reciprocal
+  // (x + 1/2 is never within rounding of a multiple)
+  if (tid < 32) {
+    int n_seg = 0, n_open = 0, tile = 0, k = 0, used = 0, weight = 0, pos0 = 0;
+    auto close = [&]() {
+      if (tid == 0) {
+        S.open_tile[n_open] = tile;
+        S.open_pos[n_open] = pos0;
+        S.open_n[n_open] = k;
       }
-      if (m > 0) {
-        const int f = m / per;
-        S.seg_tile[S.n_seg] = tile;
-        S.seg_pos[S.n_seg] = pos;
-        S.seg_per[S.n_seg] = per;
-        S.seg_n[S.n_seg++] = f;
-        tile += f;
-        pos += f * per;
-        m -= f * per;
+      ++n_open;
+      ++tile;
+      k = 0;
+    };
+    for (int c0 = 0; c0 < S.n_cls; c0 += 32) {
+      const int ci = c0 + tid, mc = ci < S.n_cls ? S.cls[ci] : 0;
+      const bool in = mc >= max(c_lo, 1) && mc <= c_hi;
+      const int mpos = in ? S.base[mc] : 0, mm = in ? min(S.cnt[mc], limit - mpos) : 0;
+      const float minv = 1.f / (float)max(mc, 1);
+      for (int l = 0; l < min(32, S.n_cls - c0); ++l) {
+        const int c = __shfl_sync(0xffffffffu, mc, l);
+        int m = __shfl_sync(0xffffffffu, mm, l), pos = __shfl_sync(0xffffffffu, mpos, l);
+        const float inv = __shfl_sync(0xffffffffu, minv, l);
+        if (m <= 0) continue;
+        const int sh = c >= dbl ? 1 : 0;
+        if (k > 0) {
+          const int r = min(m, min((int)(((float)(room - used) + 0.5f) * inv),
+                                   (most - weight) >> sh));
+          k += r;
+          used += r * c;
+          weight += r << sh;
+          pos += r;
+          m -= r;
+          if (m > 0) close();
+        }
         if (m > 0) {
-          pos0 = pos;
-          k = m;
-          used = m * c;
-          weight = m * wt;
+          const int per = min((int)(((float)room + 0.5f) * inv), most >> sh), f = m / per;
+          if (f > 0) {
+            if (tid == 0) {
+              S.seg_tile[n_seg] = tile;
+              S.seg_pos[n_seg] = pos;
+              S.seg_per[n_seg] = per;
+              S.seg_n[n_seg] = f;
+            }
+            ++n_seg;
+            tile += f;
+            pos += f * per;
+            m -= f * per;
+          }
+          if (m > 0) {
+            pos0 = pos;
+            k = m;
+            used = m * c;
+            weight = m << sh;
+          }
         }
       }
     }
-    if (k > 0) {
-      S.open_tile[S.n_open] = tile++;
-      S.open_pos[S.n_open] = pos0;
-      S.open_n[S.n_open++] = k;
+    if (k > 0) close();
+    if (tid == 0) {
+      S.n_seg = n_seg;
+      S.n_open = n_open;
+      S.n_tiles = tile;
     }
-    S.n_tiles = tile;
   }
   __syncthreads();
 }
