@@ -25,6 +25,7 @@ struct TeMma {
   int32_t* order;    // (n,) genes stably sorted by bin count (sources)
   // the rest only when cap_rows > 0
   int64_t cap_rows;  // bit-plane rows there is room for
+  int sm_pairs;      // pairs of SMs of the device
   int max_cells;     // most cells of a pair of the tensor cores (a rule on N)
   int words;         // 32-bit words of a plane row (a multiple of 8)
   int32_t* rowoff;   // (n,) by gene: first plane row, -1 without planes

@@ -1268,6 +1268,7 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   M.t_first = P.t_first;
   M.t_last = P.t_first + P.n_targets - 1;
   M.ws = P.ws;
+  M.sm_pairs = A.sm_count / 2;
   M.order = order;
   M.out_mode = out_mode;
   M.out = out;
