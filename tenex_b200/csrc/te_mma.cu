@@ -216,10 +216,16 @@ __device__ void pack_tiles(PlanShared& S, int c_lo, int c_hi, int room, int most
       const bool in = mc >= max(c_lo, 1) && mc <= c_hi;
       const int mpos = in ? S.base[mc] : 0, mm = in ? min(S.cnt[mc], limit - mpos) : 0;
       const float minv = 1.f / (float)max(mc, 1);
+      const int mper = min((int)(((float)room + 0.5f) * minv), most >> (mc >= dbl ? 1 : 0));
+      const float mpinv = 1.f / (float)max(mper, 1);
+      // full tiles' worth of members: the quotient by a reciprocal holds below 2^20
+      const bool exact = limit >= (1 << 20);
       for (int l = 0; l < min(32, S.n_cls - c0); ++l) {
         const int c = __shfl_sync(0xffffffffu, mc, l);
         int m = __shfl_sync(0xffffffffu, mm, l), pos = __shfl_sync(0xffffffffu, mpos, l);
         const float inv = __shfl_sync(0xffffffffu, minv, l);
+        const int per = __shfl_sync(0xffffffffu, mper, l);
+        const float pinv = __shfl_sync(0xffffffffu, mpinv, l);
         if (m <= 0) continue;
         const int sh = c >= dbl ? 1 : 0;
         if (k > 0) {
@@ -233,7 +239,7 @@ __device__ void pack_tiles(PlanShared& S, int c_lo, int c_hi, int room, int most
           if (m > 0) close();
         }
         if (m > 0) {
-          const int per = min((int)(((float)room + 0.5f) * inv), most >> sh), f = m / per;
+          const int f = exact ? m / per : (int)(((float)m + 0.5f) * pinv);
           if (f > 0) {
             if (tid == 0) {
               S.seg_tile[n_seg] = tile;
@@ -362,9 +368,11 @@ __global__ void __launch_bounds__(1024) plan_kernel(TeMma M) {
   }
   __syncthreads();
   pack_tiles(S, 1, kMaxCols, S.room, kSlots, kSplitCols, n, tid);
-  emit_tiles(S, [&](int t, int pos, int m) {
-    const int4 a = M.tgt[pos], b = M.tgt[pos + m - 1];
-    M.ttile[t] = make_int4(pos, m, a.z, b.z + M.ncols[b.x] - a.z);
+  emit_tiles(S, [&](int t, int pos, int m) { M.ttile[t] = make_int4(pos, m, 0, 0); }, tid);
+  for (int t = tid; t < S.n_tiles; t += 1024) {
+    const int2 pm = make_int2(M.ttile[t].x, M.ttile[t].y);
+    const int4 a = M.tgt[pm.x], b = M.tgt[pm.x + pm.y - 1];
+    M.ttile[t] = make_int4(pm.x, pm.y, a.z, b.z + M.ncols[b.x] - a.z);
     // the tile's first target has the fewest columns, so the most sources
     const int cut = a.w;
     int lo = 0, hi = n_stiles;  // source tiles that start below cut
@@ -374,7 +382,8 @@ __global__ void __launch_bounds__(1024) plan_kernel(TeMma M) {
       else hi = mid;
     }
     M.nst[t] = lo;
-  }, tid);
+  }
+  __syncthreads();
   const int n_ttiles = S.n_tiles;
   // items: block by block of kBlk pairs of source tiles, within it target tile by
   // target tile
