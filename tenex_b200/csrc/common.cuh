@@ -78,6 +78,28 @@ __device__ __forceinline__ unsigned warp_max(unsigned v) {
   return v;
 }
 
+// 1 / c of a count 1 <= c <= 2^24: the hardware's approximation and one Newton-Raphson
+// step with fused multiply-adds (P. Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990). Equal to __frcp_rn for every whole number
+// in that range (checked one by one) in a quarter of its instructions.
+__device__ __forceinline__ float rcp_count(float c) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(c));
+  return fmaf(r, fmaf(-c, r, 1.f), r);
+}
+
+// acc + c log2(c (1 / c2b) (c1 / c2a)), the cell's term, exactly acc where c c1 == c2a c2b;
+// q = {c1 / c2a, c2a}, inv = 1 / c2b. An empty cell's ratio is 0, so it takes 0 times a
+// finite logarithm. lg2.approx of a normal number, without __log2f's denormal scaling.
+__device__ __forceinline__ float add_term(float acc, float c, float c1, float c2b, float inv,
+                                          float2 q) {
+  const float x = fmaxf(c * inv * q.x, 1e-30f);
+  float t;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
+  if (c * c1 != q.y * c2b) acc = fmaf(c, t, acc);
+  return acc;
+}
+
 // Named barrier over `nthreads` threads (a multiple of 32) with id in [1, 15].
 __device__ __forceinline__ void named_bar(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

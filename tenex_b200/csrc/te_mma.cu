@@ -526,31 +526,16 @@ __device__ __forceinline__ uint4 expand_col(uint32_t m) {
 }
 
 // acc plus the sum over the L states xt1 of one xt (this lane's source bin y) of
-// te_pair.cu's terms: c log2(c (1 / c2b) (c1 / c2a)), exactly 0 where c c1 == c2a c2b.
-// The reciprocal is the hardware's approximation and one Newton-Raphson step with fused
-// multiply-adds (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990): equal to __frcp_rn for every whole number up to 2^24
-// (checked one by one), a quarter of its instructions. An empty cell has a ratio of 0,
-// so its term is 0 times a finite logarithm.
+// te_pair.cu's terms.
 template <int L, int R>
 __device__ __forceinline__ float group_terms(float acc, const uint32_t (&r)[R], const float2* q,
                                              float c1) {
   float b = __uint_as_float(r[0]);
 #pragma unroll
   for (int u = 1; u < L; ++u) b += __uint_as_float(r[u]);
-  const float d = fmaxf(b, 1.f);
-  float inv;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(d));
-  inv = fmaf(inv, fmaf(-d, inv, 1.f), inv);
+  const float inv = dev::rcp_count(fmaxf(b, 1.f));
 #pragma unroll
-  for (int u = 0; u < L; ++u) {
-    const float c = __uint_as_float(r[u]);
-    const float2 qu = q[u];
-    const float x = fmaxf(c * inv * qu.x, 1e-30f);
-    float t;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
-    if (c * c1 != qu.y * b) acc = fmaf(c, t, acc);
-  }
+  for (int u = 0; u < L; ++u) acc = dev::add_term(acc, __uint_as_float(r[u]), c1, b, inv, q[u]);
   return acc;
 }
 

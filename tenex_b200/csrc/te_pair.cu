@@ -155,6 +155,10 @@ __device__ __forceinline__ uint32_t cell_get(const uint32_t* slot, uint32_t z, u
   return slot[z * bs + y];
 }
 
+__device__ __forceinline__ void red_shared(uint32_t addr, uint32_t inc) {
+  asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(inc) : "memory");
+}
+
 // Counts one sample: one reduction per sample (inline PTX, no return value).
 // kSlot16 adds 1 or 1 << 16 to the word holding the cell's 16-bit half. base is
 // the slot's address: the 32-bit shared window address, or (kGmem, the
@@ -172,23 +176,42 @@ __device__ __forceinline__ void hist_add(uint64_t base, uint32_t z, uint32_t y, 
   if (MODE == kGmem)
     asm volatile("red.global.add.u32 [%0], %1;" ::"l"(base + off), "r"(inc) : "memory");
   else
-    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"((uint32_t)base + off), "r"(inc) : "memory");
+    red_shared((uint32_t)base + off, inc);
+}
+
+// Four samples of 1-byte target states zs and source bins ys. Shared slots: the cell's
+// address base + 4 (z row + y) is one two-way dot product of the bytes (z, y) with
+// (4 row, 4), the bytes paired by one permute per two samples: 2.5 instructions a sample
+// with the reduction, where extracting, multiplying and adding took 5 and the logic
+// pipe, at 59%, was the busiest. 16-bit halves pair z with y >> 1; the increment is
+// 1 + 0xffff (y & 1), another dot product.
+template <int MODE>
+__device__ __forceinline__ void hist4_z8(uint64_t slot, uint32_t ys, uint32_t zs, uint32_t bs,
+                                         uint32_t hb) {
+  if (MODE == kGmem) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      hist_add<MODE>(slot, __byte_perm(zs, 0, 0x4440 + b), __byte_perm(ys, 0, 0x4440 + b), bs,
+                     hb);
+    return;
+  }
+  const uint32_t base = (uint32_t)slot, row = (MODE == kSlot16 ? hb : bs) * 4u | 4u << 16;
+  const uint32_t y = MODE == kSlot16 ? (ys >> 1) & 0x7f7f7f7fu : ys;
+  const uint32_t lo = __byte_perm(zs, y, 0x5140), hi = __byte_perm(zs, y, 0x7362);
+  const uint32_t odd = ys & 0x01010101u;
+  red_shared(__dp2a_lo(row, lo, base), MODE == kSlot16 ? __dp2a_lo(0xffffu, odd, 1u) : 1u);
+  red_shared(__dp2a_hi(row, lo, base), MODE == kSlot16 ? __dp2a_lo(0xffff0000u, odd, 1u) : 1u);
+  red_shared(__dp2a_lo(row, hi, base), MODE == kSlot16 ? __dp2a_hi(0xffffu, odd, 1u) : 1u);
+  red_shared(__dp2a_hi(row, hi, base), MODE == kSlot16 ? __dp2a_hi(0xffff0000u, odd, 1u) : 1u);
 }
 
 template <int MODE>
 __device__ __forceinline__ void hist16_z8(uint64_t slot, uint4 yv, uint4 zv, uint32_t bs,
                                           uint32_t hb) {
-  const uint32_t ys[4] = {yv.x, yv.y, yv.z, yv.w};
-  const uint32_t zs[4] = {zv.x, zv.y, zv.z, zv.w};
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const uint32_t y = __byte_perm(ys[w], 0, 0x4440 + b);
-      const uint32_t z = __byte_perm(zs[w], 0, 0x4440 + b);
-      hist_add<MODE>(slot, z, y, bs, hb);
-    }
-  }
+  hist4_z8<MODE>(slot, yv.x, zv.x, bs, hb);
+  hist4_z8<MODE>(slot, yv.y, zv.y, bs, hb);
+  hist4_z8<MODE>(slot, yv.z, zv.z, bs, hb);
+  hist4_z8<MODE>(slot, yv.w, zv.w, bs, hb);
 }
 
 // Same for a group whose target states were sorted at staging (sort_state_groups):
@@ -202,7 +225,6 @@ template <int MODE>
 __device__ __forceinline__ void hist16_z8_sorted(uint64_t slot, uint4 yv, uint4 zv, uint2 pm,
                                                  uint32_t bs, uint32_t hb) {
   const uint32_t zs[4] = {zv.x, zv.y, zv.z, zv.w};
-  uint32_t ys[4];
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
     const uint32_t nib = ((w < 2 ? pm.x : pm.y) >> (16 * (w & 1))) & 0xffffu;
@@ -210,33 +232,44 @@ __device__ __forceinline__ void hist16_z8_sorted(uint64_t slot, uint4 yv, uint4 
     const uint32_t sb = 0x3210u | ((nib & 0x8888u) >> 1);  // low (i) or high (i + 4) pair
     const uint32_t lo = __byte_perm(yv.x, yv.y, sa);
     const uint32_t hi = __byte_perm(yv.z, yv.w, sa);
-    ys[w] = __byte_perm(lo, hi, sb);
-  }
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const uint32_t y = __byte_perm(ys[w], 0, 0x4440 + b);
-      const uint32_t z = __byte_perm(zs[w], 0, 0x4440 + b);
-      hist_add<MODE>(slot, z, y, bs, hb);
-    }
+    hist4_z8<MODE>(slot, __byte_perm(lo, hi, sb), zs[w], bs, hb);
   }
 }
 
+// Two-byte target states: 4 y + base and then 4 row z as two dot products a sample, for
+// rows of at most 63 words (every coarsened input; their four-fold must fit a byte).
 template <int MODE>
 __device__ __forceinline__ void hist16_z16(uint64_t slot, uint4 yv, uint4 za, uint4 zb,
                                            uint32_t bs, uint32_t hb) {
   const uint32_t ys[4] = {yv.x, yv.y, yv.z, yv.w};
   const uint32_t zs[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
+  const uint32_t row = (MODE == kSlot16 ? hb : bs) * 4u;
+  if (MODE == kGmem || row > 255u) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const uint32_t y = __byte_perm(ys[w], 0, 0x4440 + b);
+        const uint32_t zw = zs[(w * 4 + b) >> 1];
+        const uint32_t z = (b & 1) ? (zw >> 16) : (zw & 0xffffu);
+        hist_add<MODE>(slot, z, y, bs, hb);
+      }
+    }
+    return;
+  }
+  const uint32_t base = (uint32_t)slot, rows = row | row << 24;
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const uint32_t y = __byte_perm(ys[w], 0, 0x4440 + b);
-      const uint32_t zw = zs[(w * 4 + b) >> 1];
-      const uint32_t z = (b & 1) ? (zw >> 16) : (zw & 0xffffu);
-      hist_add<MODE>(slot, z, y, bs, hb);
-    }
+    const uint32_t y = MODE == kSlot16 ? (ys[w] >> 1) & 0x7f7f7f7fu : ys[w];
+    const uint32_t odd = ys[w] & 0x01010101u, z0 = zs[2 * w], z1 = zs[2 * w + 1];
+    red_shared(__dp2a_lo(z0, rows, __dp4a(y, 4u, base)),
+               MODE == kSlot16 ? __dp2a_lo(0xffffu, odd, 1u) : 1u);
+    red_shared(__dp2a_hi(z0, rows, __dp4a(y, 4u << 8, base)),
+               MODE == kSlot16 ? __dp2a_lo(0xffff0000u, odd, 1u) : 1u);
+    red_shared(__dp2a_lo(z1, rows, __dp4a(y, 4u << 16, base)),
+               MODE == kSlot16 ? __dp2a_hi(0xffffu, odd, 1u) : 1u);
+    red_shared(__dp2a_hi(z1, rows, __dp4a(y, 4u << 24, base)),
+               MODE == kSlot16 ? __dp2a_hi(0xffff0000u, odd, 1u) : 1u);
   }
 }
 
@@ -331,42 +364,35 @@ __device__ __forceinline__ float entropy_cols(uint32_t* tab, int bt, int bs, int
   // every word of a row, padding included (zero, so skipped by the s == 0 test):
   // consecutive lanes then read consecutive words, one wavefront per warp
   const int ncy = stride;
-  const int ncols = bt * ncy;
+  const int ncols = bt * ncy, step = bt * stride;  // words between the states xt1 of a column
   for (int col = lane_g; col < ncols; col += gthreads) {
     const int j = col / ncy;
-    const int wk = col - j * ncy;
+    uint32_t* p = tab + col;  // cell (0, xt = j, y): word j * stride + y
     uint32_t s = 0;
-    for (int i = 0; i < bt; ++i) s += tab[(i * bt + j) * stride + wk];
+#pragma unroll 4
+    for (int i = 0; i < bt; ++i) s += p[i * step];
     if (s == 0u) continue;
     const float c1j = (float)c1i[j];
+    const float2* q = qa + j;  // {c1/c2a, c2a}
     if (PACK16) {
       const float blo = (float)(s & 0xffffu), bhi = (float)(s >> 16);
-      const float inv_lo = __frcp_rn(blo), inv_hi = __frcp_rn(bhi);
-      for (int i = 0; i < bt; ++i) {
-        const int idx = (i * bt + j) * stride + wk;
-        const uint32_t w = tab[idx];
-        if (CLEAR) tab[idx] = 0u;
-        const float2 q = qa[i * bt + j];  // {c1/c2a, c2a}
-        const float clo = (float)(w & 0xffffu), chi = (float)(w >> 16);
-        const bool elo = clo == 0.f || clo * c1j == q.y * blo;
-        const bool ehi = chi == 0.f || chi * c1j == q.y * bhi;
-        const float rlo = elo ? 1.f : clo * inv_lo * q.x;
-        const float rhi = ehi ? 1.f : chi * inv_hi * q.x;
-        acc = fmaf(clo, __log2f(rlo), acc);
-        acc = fmaf(chi, __log2f(rhi), acc);
+      const float inv_lo = dev::rcp_count(fmaxf(blo, 1.f));
+      const float inv_hi = dev::rcp_count(fmaxf(bhi, 1.f));
+#pragma unroll 4
+      for (int i = 0; i < bt; ++i, p += step, q += bt) {
+        const uint32_t w = *p;
+        if (CLEAR) *p = 0u;
+        acc = dev::add_term(acc, (float)(w & 0xffffu), c1j, blo, inv_lo, *q);
+        acc = dev::add_term(acc, (float)(w >> 16), c1j, bhi, inv_hi, *q);
       }
     } else {
       const float b = (float)s;
-      const float inv = __frcp_rn(b);
-      for (int i = 0; i < bt; ++i) {
-        const int idx = (i * bt + j) * stride + wk;
-        const uint32_t w = tab[idx];
-        if (CLEAR) tab[idx] = 0u;
-        const float2 q = qa[i * bt + j];
-        const float c = (float)w;
-        const bool e = w == 0u || c * c1j == q.y * b;
-        const float r = e ? 1.f : c * inv * q.x;
-        acc = fmaf(c, __log2f(r), acc);
+      const float inv = dev::rcp_count(b);
+#pragma unroll 4
+      for (int i = 0; i < bt; ++i, p += step, q += bt) {
+        const uint32_t w = *p;
+        if (CLEAR) *p = 0u;
+        acc = dev::add_term(acc, (float)w, c1j, b, inv, *q);
       }
     }
   }
