@@ -674,6 +674,7 @@ __device__ __forceinline__ void run_sources(const TeParams& P, const ItemCtx& it
   const int N = P.N;
   const uint64_t slot_addr = table_addr<MODE>(slot, tid);
   if (P.ztile >= N) {
+    if (g >= n_groups) return;  // a warp without a slot
     for (int r = g; r < it.n_src; r += n_groups) {
       int src;
       int64_t p;
@@ -693,7 +694,7 @@ __device__ __forceinline__ void run_sources(const TeParams& P, const ItemCtx& it
   for (int r0 = 0; r0 < it.n_src; r0 += n_groups) {
     int src = 0;
     int64_t p = 0;
-    const bool act = r0 + g < it.n_src && pair_of<MODE>(P, it, r0 + g, &src, &p);
+    const bool act = g < n_groups && r0 + g < it.n_src && pair_of<MODE>(P, it, r0 + g, &src, &p);
     float obs_m = 0.f;
     if (act && P.out_mode == kOutStats && lane_g == 0)
       obs_m = __ldg(P.obs + (int64_t)src * P.n + it.tgt);
@@ -892,9 +893,9 @@ __global__ void __launch_bounds__(1024, 1) te_pair_tile_kernel(TeParams P) {
       continue;
     }
     int G = 1;
-    while (n_warps / G > fit) G <<= 1;
-    while (G > 1 && G < n_warps && n_warps / G > 15) G <<= 1;
-    const int n_groups = n_warps / G;
+    while (G < n_warps && min(n_warps / G, fit) * G * 4 < n_warps * 3) G <<= 1;
+    while (G > 1 && G < n_warps && 15 * G * 2 < n_warps) G <<= 1;
+    const int n_groups = min(min(n_warps / G, fit), G > 1 ? 15 : n_warps);
     // odd row stride where the same groups' slots still fit at the padded size
     // (the group size and the counter width stay as chosen above)
     bool pad = false;
