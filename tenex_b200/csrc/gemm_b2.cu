@@ -120,9 +120,12 @@ __device__ __forceinline__ void tmem_wait_ld() {
 // (4 reciprocals, 8 logarithms) instead of a division per cell.
 __device__ __forceinline__ float cell_term(float c, float c1, float c2a, float c2b, float q,
                                            float rb) {
-  const bool e = c == 0.f || c * c1 == c2a * c2b;
-  const float r = e ? 1.f : c * rb * q;
-  return c * __log2f(r);
+  // an empty cell's ratio is 0 or a NaN (fmaxf returns the other operand): its term is 0
+  // times a finite logarithm; a normal number's lg2.approx without denormal scaling
+  const float x = fmaxf(c * rb * q, 1e-30f);
+  float t;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
+  return c * c1 == c2a * c2b ? 0.f : c * t;
 }
 
 // Pack: F[g, t] = x[g, t+lag] (the lag-shifted operand TMA cannot address: its
@@ -437,51 +440,61 @@ __global__ void __launch_bounds__(B2Layout<TN>::kThreads, B2Layout<TN>::kCtasPer
     }
   }
 
-  // ---- MMA issuer (warp 1, lane 0): stage k's MMAs as soon as its operands are
-  // in place; never waits on MMA completion, so the tensor pipe gets the stages
-  // back to back. The source tile P_j is the A operand (M = 128 lanes = sources)
-  // and the target tiles are B: [FP_i; P_i] (adjacent in the stage, one N = 256
-  // MMA) and F_i (N = 128), so a K step reads P_j twice instead of three times
-  // (20 KB of shared memory instead of 24 at TN = 128). TMEM columns 0..TN-1 =
-  // C^T, TN..2TN-1 = D^T, 256..256+TN-1 = E^T.
-  if (tid == 32) {
+  // ---- MMA issuer (warp 1): stage k's MMAs as soon as its operands are in place;
+  // never waits on MMA completion, so the tensor pipe gets the stages back to back.
+  // The whole warp runs the loop and one elected lane issues, so that descriptors are
+  // sums of a base and constants in uniform registers: with one lane running it, building
+  // them took longer than the MMAs (2,000 x 5,000: 50 -> 47 us). The source tile P_j is
+  // the A operand (M = 128 lanes = sources) and the target tiles are B: [FP_i; P_i]
+  // (adjacent in the stage, one N = 256 MMA) and F_i (N = 128), so a K step reads P_j
+  // twice instead of three times (20 KB of shared memory instead of 24 at TN = 128).
+  // TMEM columns 0..TN-1 = C^T, TN..2TN-1 = D^T, 256..256+TN-1 = E^T.
+  if (warp == 1) {
     const uint32_t idesc256 = FP4 ? idesc_mxf4(kTile, 2 * TN) : idesc_i8(kTile, 2 * TN);
     const uint32_t idesc128 = FP4 ? idesc_mxf4(kTile, TN) : idesc_i8(kTile, TN);
+    const uint32_t desc0 = (uint32_t)smem_desc_sw128(smem_u32(stage_base));  // low word
+    const bool elected = elect_one();
     bool ok = true;
+    uint32_t s = 0, ph = 0;
     for (int k = 0; k < nk; ++k) {
-      const int s = k % kStages;
-      const uint32_t ph = (uint32_t)((k / kStages) & 1);
       if (*(volatile int*)abort_flag || !mbar_wait(&full[s], ph)) {
         ok = false;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      unsigned char* buf = stage_base + s * kStageBytes;
-      const uint32_t bFPP = smem_u32(buf + 0 * kTgtBytes);  // FP_i rows, then P_i rows
-      const uint32_t bF = smem_u32(buf + 2 * kTgtBytes);
-      const uint32_t aPj = smem_u32(buf + 3 * kTgtBytes);
+      // FP_i rows, P_i rows, F_i rows, then P_j rows
+      const uint32_t bFPP = desc0 + s * (uint32_t)(kStageBytes >> 4);
+      const uint32_t bF = bFPP + (uint32_t)(2 * kTgtBytes >> 4);
+      const uint32_t aPj = bFPP + (uint32_t)(3 * kTgtBytes >> 4);
+      if (elected) {
 #pragma unroll
-      for (int kk = 0; kk < kKt / 32; ++kk) {
-        const uint32_t off = kk * 32;  // 32-byte K step inside the 128-byte swizzle row
-        const uint64_t ad = smem_desc_sw128(aPj + off);
-        const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
-        if (FP4) {
-          mma_mxf4(tmem + 0, ad, smem_desc_sw128(bFPP + off), idesc256, acc, tmem + kSfaCol,
-                   tmem + kSfbCol);
-          mma_mxf4(tmem + kECol, ad, smem_desc_sw128(bF + off), idesc128, acc, tmem + kSfaCol,
-                   tmem + kSfbCol);
-        } else {
-          mma_i8(tmem + 0, ad, smem_desc_sw128(bFPP + off), idesc256, acc);
-          mma_i8(tmem + kECol, ad, smem_desc_sw128(bF + off), idesc128, acc);
+        for (uint32_t kk = 0; kk < kKt / 32; ++kk) {
+          // 32-byte K step inside the 128-byte swizzle row: 2 in a descriptor's address
+          const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
+          if (FP4) {
+            mma_mxf4_lo(tmem + 0, aPj + 2 * kk, bFPP + 2 * kk, idesc256, acc, tmem + kSfaCol,
+                        tmem + kSfbCol);
+            mma_mxf4_lo(tmem + kECol, aPj + 2 * kk, bF + 2 * kk, idesc128, acc, tmem + kSfaCol,
+                        tmem + kSfbCol);
+          } else {
+            mma_i8_lo(tmem + 0, aPj + 2 * kk, bFPP + 2 * kk, idesc256, acc);
+            mma_i8_lo(tmem + kECol, aPj + 2 * kk, bF + 2 * kk, idesc128, acc);
+          }
         }
+        mma_commit(&empty[s]);  // stage s free once these MMAs complete
       }
-      mma_commit(&empty[s]);  // stage s free once these MMAs complete
+      __syncwarp();
+      if (++s == kStages) {
+        s = 0;
+        ph ^= 1;
+      }
     }
-    if (!ok) {
+    if (!ok && elected) {
       atomicExch(prm.err, 1);
       *(volatile int*)abort_flag = 1;
     }
-    mma_commit(accbar);  // arrives after every issued MMA, so the epilogue wakes either way
+    if (elected) mma_commit(accbar);  // after every issued MMA, so the epilogue wakes either way
+    __syncwarp();
   }
 
   // ---- epilogue: every warp; lane quarter warp % 4, column group warp / 4 -----

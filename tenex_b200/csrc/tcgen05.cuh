@@ -133,6 +133,37 @@ __device__ __forceinline__ void mma_mxf4(uint32_t d_tmem, uint64_t adesc, uint64
       : "memory");
 }
 
+// High word of every smem_desc_sw128 descriptor (SBO, version, swizzle): the low word
+// alone tells the operand's address.
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+
+// mma_i8 and mma_mxf4 with the low words of smem_desc_sw128 descriptors.
+__device__ __forceinline__ void mma_i8_lo(uint32_t d_tmem, uint32_t a, uint32_t b, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 ad, {%1, %5};\n\t"
+      "mov.b64 bd, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], ad, bd, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(kDescHigh)
+      : "memory");
+}
+
+__device__ __forceinline__ void mma_mxf4_lo(uint32_t d_tmem, uint32_t a, uint32_t b,
+                                            uint32_t idesc, uint32_t accumulate, uint32_t sfa,
+                                            uint32_t sfb) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 ad, {%1, %7};\n\t"
+      "mov.b64 bd, {%2, %7};\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], ad, bd, %3, [%5], [%6], "
+      "p;\n\t}" ::"r"(d_tmem),
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb), "r"(kDescHigh)
+      : "memory");
+}
+
 // Stores v into 8 consecutive TMEM columns starting at taddr for the 32 lanes of
 // the calling warp's lane quarter (taddr's lane field = 32 * (warp % 4)).
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, uint32_t v) {
@@ -203,7 +234,6 @@ __device__ __forceinline__ bool elect_one() {
 // unit scale factors of both operands.
 __device__ __forceinline__ void mma_mxf4_pair(uint32_t d_tmem, uint32_t a, uint32_t b,
                                               uint32_t idesc, uint32_t accumulate, uint32_t sf) {
-  constexpr uint32_t kHigh = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO, version, swizzle
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
@@ -211,7 +241,7 @@ __device__ __forceinline__ void mma_mxf4_pair(uint32_t d_tmem, uint32_t a, uint3
       "mov.b64 bd, {%2, %6};\n\t"
       "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], ad, bd, %3, [%5], [%5], "
       "p;\n\t}" ::"r"(d_tmem),
-      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(sf), "r"(kHigh)
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(sf), "r"(kDescHigh)
       : "memory");
 }
 
