@@ -7,6 +7,8 @@
 
 #include <mutex>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace tenex {
@@ -100,6 +102,78 @@ __global__ void block_shuffle_kernel(const uint8_t* __restrict__ in, int64_t in_
     *reinterpret_cast<uint4*>(dst + i0) = make_uint4(w[0], w[1], w[2], w[3]);
   } else {
     for (uint32_t u = 0; i0 + u < row; ++u) dst[i0 + u] = (uint8_t)(w[u >> 2] >> (8u * (u & 3u)));
+  }
+}
+
+// The same with a gene's row in shared memory, for blocks of 16 bytes or more: one CTA
+// per gene and group of `per` copies reads the row once. 16 output bytes then come from
+// at most two places of the row, five aligned words each, put together by funnel shifts
+// and merged at the block's end. 2,000 genes x 100 copies of 5,000 bytes (1 GB written):
+// 2.37 -> 1.09 ms; the kernel above gathers byte by byte from global memory.
+constexpr uint32_t kShufflePad = 32;  // zero bytes before and after the row
+__global__ void __launch_bounds__(256) block_shuffle_row_kernel(
+    const uint8_t* __restrict__ in, int64_t in_ld, uint32_t row, uint32_t blK, uint32_t head,
+    const int32_t* __restrict__ perm, int64_t perm_stride, int n_blocks, int copies, int per,
+    uint8_t* __restrict__ out, int64_t out_ld, int64_t out_stride) {
+  extern __shared__ __align__(16) unsigned char sh[];
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(sh);
+  const int g = blockIdx.x;
+  const uint8_t* src = in + (int64_t)g * in_ld;
+  for (uint32_t i = threadIdx.x; i < row + 2 * kShufflePad; i += blockDim.x)
+    sh[i] = i >= kShufflePad && i < row + kShufflePad ? src[i - kShufflePad] : 0;
+  __syncthreads();
+  // 16 bytes of the row from byte j >= -16 on
+  auto take = [&](int j, uint32_t (&w)[4]) {
+    const uint32_t at = (uint32_t)(j + (int)kShufflePad), shift = (at & 3u) * 8u;
+    const uint32_t* p = words + (at >> 2);
+    uint32_t a = p[0];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t b = p[u + 1];
+      w[u] = __funnelshift_r(a, b, shift);
+      a = b;
+    }
+  };
+  const int c0 = blockIdx.y * per, c1 = min(copies, c0 + per);
+  for (uint32_t i0 = threadIdx.x * 16u; i0 < row; i0 += blockDim.x * 16u) {
+    const uint32_t b = i0 / blK, off = i0 - b * blK;
+    const bool in1 = i0 < head;
+    const uint32_t len = in1 ? min(16u, blK - off) : 16u;  // bytes of the first place
+    const bool two = len < 16u, in2 = i0 + len < head;
+    uint32_t mask[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+      const int k = (int)len - 4 * (int)u;  // of this word's bytes
+      mask[u] = k >= 4 ? 0xffffffffu : k <= 0 ? 0u : (1u << (8 * k)) - 1u;
+    }
+    for (int c = c0; c < c1; ++c) {
+      const int32_t* pg = perm + (int64_t)c * perm_stride + (int64_t)g * n_blocks;
+      uint32_t j = i0;
+      if (in1) {
+        uint32_t pb = (uint32_t)__ldg(pg + b);
+        if (pb >= (uint32_t)n_blocks) pb = b;  // out-of-range entry: identity
+        j = pb * blK + off;
+      }
+      uint32_t w[4];
+      take((int)j, w);
+      if (two) {
+        uint32_t j2 = i0 + len, w2[4];
+        if (in2) {
+          uint32_t pb = (uint32_t)__ldg(pg + b + 1);
+          if (pb >= (uint32_t)n_blocks) pb = b + 1;
+          j2 = pb * blK;
+        }
+        take((int)j2 - (int)len, w2);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = (w[u] & mask[u]) | (w2[u] & ~mask[u]);
+      }
+      uint8_t* dst = out + (int64_t)c * out_stride + (int64_t)g * out_ld + i0;
+      if (i0 + 16u <= row) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+        for (uint32_t u = 0; i0 + u < row; ++u) dst[u] = (uint8_t)(w[u >> 2] >> (8u * (u & 3u)));
+      }
+    }
   }
 }
 
@@ -202,6 +276,26 @@ extern "C" int tenex_block_shuffle_many(const uint8_t* in, int64_t in_ld, int n_
   const int64_t gx = (row + 4095) / 4096;
   if (n_vars > 65535 || n_copies > 65535)
     return fail(TENEX_ERR_UNSUPPORTED, "grid too large (n_vars=%d, copies=%d)", n_vars, n_copies);
+  // several copies, rows that fit shared memory next to a second CTA, blocks of 16 bytes
+  // or more (one copy: 10.8 us by the kernel above, 13.9 by this one, 1,000 x 5,000)
+  const int64_t sh = row + 2 * kShufflePad;
+  if (n_copies > 1 && (int64_t)block_length * K >= 16 && sh <= 100 * 1024) {
+    DevAttr A;
+    const int st = current_device_attr(&A);
+    if (st) return st;
+    // every copy in one CTA unless that leaves fewer than eight CTAs per SM
+    const int groups = std::max(1, std::min(n_copies, 8 * A.sm_count / n_vars));
+    const int per = (n_copies + groups - 1) / groups;
+    cudaError_t e = cudaFuncSetAttribute(block_shuffle_row_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute");
+    block_shuffle_row_kernel<<<dim3((unsigned)n_vars, (unsigned)((n_copies + per - 1) / per)),
+                               256, (size_t)sh, as_stream(stream)>>>(
+        in, in_ld, (uint32_t)row, (uint32_t)(block_length * K),
+        (uint32_t)((int64_t)n_blocks * block_length * K), perms, (int64_t)n_vars * n_blocks,
+        n_blocks, n_copies, per, out, out_ld, out_copy_stride);
+    return check_launch("block_shuffle_row_kernel");
+  }
   dim3 grid((unsigned)gx, (unsigned)n_vars, (unsigned)n_copies);
   block_shuffle_kernel<<<grid, 256, 0, as_stream(stream)>>>(
       in, in_ld, n_vars, (uint32_t)row, (uint32_t)(block_length * K),
