@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from tenex_b200 import _log, native
-from tenex_b200.inference.grn import bh_fdr_gpu, build_pairs, make_grn
+from tenex_b200.inference.grn import build_pairs, make_grn
 from tenex_b200.kernels import device as D
 
 
@@ -30,9 +30,20 @@ def fdr_threshold_gpu(te: torch.Tensor, pairs: torch.Tensor, fdr: float):
         return torch.empty(0, device=te.device), pairs[:0]
     z = (te - te.mean()) / std
     pval = 0.5 * torch.erfc(z / 1.4142135623730951)
-    adj = bh_fdr_gpu(pval, 0.05)
-    mask = adj < fdr
-    return te[mask], pairs[mask]
+    # adjusted p < fdr holds for the K smallest p-values, K the last rank with
+    # p_(K) m / K < fdr, ties included: one sort of the values instead of a sort with
+    # indices, a running minimum and a scatter back
+    m = pval.shape[0]
+    if m == 0:
+        return te, pairs[:0]
+    ordered = pval.sort().values
+    rank = torch.arange(1, m + 1, device=pval.device, dtype=pval.dtype)
+    ok = (ordered * m / rank).clamp(max=1.0) < fdr
+    last = ok.nonzero()[-1:, 0]                      # empty when no p-value passes
+    if last.numel() == 0:
+        return te[:0], pairs[:0]
+    idx = (pval <= ordered[last]).nonzero(as_tuple=True)[0]
+    return te[idx], pairs[idx]
 
 
 class _LazyPairs:
@@ -57,8 +68,10 @@ class _LazyPairs:
 
 
 def _offdiag(M: torch.Tensor):
+    # the off-diagonal cells of a row-major (n, n) matrix are flat positions 1.. cut into
+    # n - 1 rows of n + 1, without each row's last
     n = M.shape[0]
-    te = M[~torch.eye(n, dtype=torch.bool, device=M.device)]
+    te = M.reshape(-1)[1:].view(max(n - 1, 0), n + 1)[:, :n].reshape(-1)
     return te, _LazyPairs(n, M.device)
 
 

@@ -467,7 +467,9 @@ def fallback_surrogates_batched(db: D.DeviceBins, npv: torch.Tensor, b_max: int,
     lag = tau * db.K
     for k0 in range(0, S, chunk):
         kk = min(chunk, S - k0)
-        big = D.empty_bins(kk * n, db.T, db.K, dev)
+        # the shuffle writes every sample of every row; nothing reads a row's padding
+        big = D.DeviceBins(torch.empty((kk * n, db.ld), dtype=torch.uint8, device=dev), kk * n,
+                           db.T, db.K)
         D.block_shuffle_many(db, perms[k0:k0 + kk], bl, big)
         off = torch.arange(kk, device=dev, dtype=torch.int64)
         pairs_big = (sp_d[None, :, :] + (off * n)[:, None, None]).reshape(-1, 2).contiguous()
