@@ -112,21 +112,12 @@ __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// c * log2(c * c1 / (c2a * c2b)); exactly 0 for an empty cell and where the two
-// products are equal (the reference's ratio is exactly 1 there); otherwise the
-// ratio as c * (1/c2b) * (c1/c2a), with q = c1/c2a divided once per target state
-// and rb = 1/c2b once per source state (approximate reciprocal, 1 ulp), and
+// The terms are dev::add_term's: c * log2(c * c1 / (c2a * c2b)), exactly 0 for an empty
+// cell and where the two products are equal (the reference's ratio is exactly 1 there);
+// otherwise the ratio as c * (1/c2b) * (c1/c2a), with q = c1/c2a divided once per target
+// state and rb = 1/c2b once per source state (approximate reciprocal, 1 ulp), and
 // lg2.approx: far below the 1e-6 TE budget, and 12 MUFU operations per pair
 // (4 reciprocals, 8 logarithms) instead of a division per cell.
-__device__ __forceinline__ float cell_term(float c, float c1, float c2a, float c2b, float q,
-                                           float rb) {
-  // an empty cell's ratio is 0 or a NaN (fmaxf returns the other operand): its term is 0
-  // times a finite logarithm; a normal number's lg2.approx without denormal scaling
-  const float x = fmaxf(c * rb * q, 1e-30f);
-  float t;
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
-  return c * c1 == c2a * c2b ? 0.f : c * t;
-}
 
 // Pack: F[g, t] = x[g, t+lag] (the lag-shifted operand TMA cannot address: its
 // copies start on 16-byte boundaries) and FP = F & P for t < L (0 beyond, up to
@@ -288,15 +279,15 @@ __device__ __forceinline__ float b2_pair_te(float C, float Dv, float E, int ti, 
   const float rb11 = __fdividef(1.f, c2b11), rb01 = __fdividef(1.f, c2b01),
               rb10 = __fdividef(1.f, c2b10), rb00 = __fdividef(1.f, c2b00);
   float te = 0.f;
-  te += cell_term(C, c1_1, c2a11, c2b11, q11, rb11);                                // [1,1,1]
-  te += cell_term(Dv - C, c1_1, c2a01, c2b11, q01, rb11);                           // [0,1,1]
-  te += cell_term(E - C, c1_0, c2a10, c2b01, q10, rb01);                            // [1,0,1]
-  te += cell_term(npj - Dv - E + C, c1_0, c2a00, c2b01, q00, rb01);                 // [0,0,1]
-  te += cell_term(nfp - C, c1_1, c2a11, c2b10, q11, rb10);                          // [1,1,0]
-  te += cell_term(np_ - Dv - nfp + C, c1_1, c2a01, c2b10, q01, rb10);               // [0,1,0]
-  te += cell_term(nf - E - nfp + C, c1_0, c2a10, c2b00, q10, rb00);                 // [1,0,0]
-  te += cell_term(N - nf - np_ - npj + nfp + Dv + E - C, c1_0, c2a00, c2b00, q00,
-                  rb00);                                                            // [0,0,0]
+  te = dev::add_term(te, C, c1_1, c2b11, rb11, make_float2(q11, c2a11));  // [1,1,1]
+  te = dev::add_term(te, Dv - C, c1_1, c2b11, rb11, make_float2(q01, c2a01));  // [0,1,1]
+  te = dev::add_term(te, E - C, c1_0, c2b01, rb01, make_float2(q10, c2a10));  // [1,0,1]
+  te = dev::add_term(te, npj - Dv - E + C, c1_0, c2b01, rb01, make_float2(q00, c2a00));  // [0,0,1]
+  te = dev::add_term(te, nfp - C, c1_1, c2b10, rb10, make_float2(q11, c2a11));  // [1,1,0]
+  te = dev::add_term(te, np_ - Dv - nfp + C, c1_1, c2b10, rb10, make_float2(q01, c2a01));  // [0,1,0]
+  te = dev::add_term(te, nf - E - nfp + C, c1_0, c2b00, rb00, make_float2(q10, c2a10));  // [1,0,0]
+  te = dev::add_term(te, N - nf - np_ - npj + nfp + Dv + E - C, c1_0, c2b00, rb00,
+                     make_float2(q00, c2a00));                                          // [0,0,0]
   return te;
 }
 

@@ -77,20 +77,22 @@ def remap_bins(raw, K: int = 1, device=None) -> tuple[D.DeviceBins, torch.Tensor
     n, row = (int(s) for s in t.shape)
     if row % K:
         raise ValueError(f"row length {row} is not a multiple of K={K}")
-    npv = torch.empty(n, dtype=torch.int32, device=dev)
-    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    # the bin counts and, behind them, the kernel's error word: one copy to the host
+    buf = torch.zeros(n + 1, dtype=torch.int32, device=dev)
+    npv, err = buf[:n], buf[n:]
     db = None
     for wide in (False, True):
         # uint8 rows; a gene with more than 256 distinct values keeps uint16 rows
         # (the reference's int16 bins, tenex/preprocess.py:335-354) until the
         # coarsening step narrows them
         db = D.empty_bins(n, row // K, K, dev, wide=wide)
-        err.zero_()
+        if wide:
+            err.zero_()
         native.call("tenex_remap_dense", t.data_ptr(), in_bytes, row, n, row,
                     db.data.data_ptr(), 2 if wide else 1, db.ld, npv.data_ptr(), err.data_ptr(),
                     native.stream_ptr())
-        # the error word and b_max come back in one copy (one wait on the stream)
-        e, b_max = (int(v) for v in torch.stack((err[0], npv.max())).cpu())
+        host = buf.cpu().numpy()
+        e, b_max = int(host[n]), int(host[:n].max(initial=0))
         if e == 1:
             raise ValueError("a gene's raw bins span more than 8192 values; cannot remap")
         if e == 0:

@@ -29,6 +29,8 @@ import torch
 from tenex_b200 import _log
 from tenex_b200.kernels import compute_smem_bytes, query_smem_optin
 from tenex_b200.kernels import device as D
+from tenex_b200.kernels.adaptive_smem import compute_smem_bin_limit
+from tenex_b200.kernels.pair_tile import PairTileKernel
 from tenex_b200.preprocess import compact_dtype, discretize
 from tenex_b200.result import TransferEntropyResult
 
@@ -265,9 +267,13 @@ class TransferEntropyEngine:
             self._finish(info, db, npv, b_max, ev, stream, t0, "matrix")
             return self._wrap_result()
 
-        # prepare (coarsening) works on a copy so the cached bins stay intact
-        work = D.DeviceBins(db.data.clone(), db.n, db.T, db.K)
-        npv_w = npv.clone()
+        # prepare (coarsening) works on a copy so the cached bins stay intact; this
+        # package's kernels leave bins of at most the bin limit as they are
+        if isinstance(kobj, PairTileKernel) and b_max <= compute_smem_bin_limit(smem_optin):
+            work, npv_w = db, npv
+        else:
+            work = D.DeviceBins(db.data.clone(), db.n, db.T, db.K)
+            npv_w = npv.clone()
         work, npv_w, b_max_w = kobj.prepare(work, npv_w, b_max, use_coarsening=coarsening,
                                             on_cuda=True, n_vars=n_vars, tau=tau,
                                             smem_optin=smem_optin)
@@ -364,7 +370,9 @@ class TransferEntropyEngine:
         # the compact dtype is applied on the device (bins are < 256, so the values
         # are unchanged), then one staged copy
         dt = torch.from_numpy(np.empty(0, dtype=compact_dtype(b_max))).dtype
-        self._last_bin_arrs = D.to_host(db.unpadded().to(dt))
+        bins = db.unpadded()
+        self._last_bin_arrs = D.to_host(bins.view(dt) if dt == torch.int8 and not db.wide
+                                        else bins.to(dt))
         self._last_n_per_var = npv.cpu().numpy()
         elapsed = time.time() - t0
         _log.vprint(f"[TENEX] done -- {elapsed:.3f}s "
