@@ -64,7 +64,8 @@ typedef struct {
 typedef struct {
   int threads;      /* threads per CTA: 128, 256, 512 or 1024          */
   int ctas_per_sm;  /* resident CTAs per SM (grid = sm_count * this)    */
-  int src_chunk;    /* sources per work item (one target per item)     */
+  int src_chunk;    /* sources per work item (one target per item);
+                       0: n_vars / 12, at least 32 and at most 512     */
   int smem_bytes;   /* dynamic shared memory per CTA (0 = fill the SM)  */
 } tenex_te_config;
 
@@ -94,7 +95,8 @@ size_t tenex_te_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 /* The launch shape the histogram kernels would use on the current device for
  * rows of row_len samples at this lag and b_max, with cfg as given (NULL or 0
  * fields: the defaults above): threads per CTA, CTAs per SM, dynamic shared
- * memory per CTA and sources per item. Same planner as the launches. */
+ * memory per CTA and sources per item (by default the most, 512). Same planner as the
+ * launches. */
 int tenex_te_launch_shape(int64_t row_len, int64_t lag, int b_max, const tenex_te_config* cfg,
                           int* threads, int* ctas_per_sm, int* smem_bytes, int* src_chunk);
 

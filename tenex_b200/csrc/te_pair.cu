@@ -1187,16 +1187,21 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   P.lag = (int)lag;
   P.p0 = p0;
   P.p1 = p0 + n_pairs;
-  // 512 sources per item: fewer target stagings than 128 (3% faster at 10,000
-  // genes), and a chunk of 512 source rows still fits L2 beside the others. Fewer where
-  // there are too few targets for 16 items per CTA (few genes, a short pair range): the
-  // items are uneven, and one round of them leaves most SMs idle at its end
-  // (301 genes x 101,003 samples: 1.88 -> 0.64 ms for the pairs counted here).
+  // Sources per item: a twelfth of them (32 at least, 512 at most). Sources are ordered
+  // by bin count and an item's slots are sized for its widest source, so a chunk should
+  // span few bin counts; below 100 sources the target's staging shows, above 512 the rows
+  // of a chunk no longer share L2. Measured at 512 / 250 / this rule, ms: 1,000 x 5,000
+  // (b to 32) 8.89 / 7.88 / 7.3, 2,000 x 5,000 (b to 16) 7.35 / 7.19 / 7.15, 2,500 x
+  // 10,000 (b to 32) 55.0 / 53.7 / 53.7; 10,000 x 20,000 at 256 / 512 / 768: 643 / 635 /
+  // 638. Fewer still where there are too few targets for 16 items per CTA (few genes, a
+  // short pair range): the items are uneven, and one round of them leaves most SMs idle
+  // at its end (301 genes x 101,003 samples: 1.88 -> 0.64 ms for the pairs counted here).
   P.W = (cfg && cfg->src_chunk) ? cfg->src_chunk : 512;
   if (!pairs && !(cfg && cfg->src_chunk)) {
     const int64_t targets = (p0 + n_pairs - 1) / (n - 1) - p0 / (n - 1) + 1;
-    const int64_t chunks = std::min<int64_t>((n + 31) / 32, 32 * A.sm_count / targets);
-    if (chunks > 1) P.W = (int)std::min<int64_t>(P.W, (n + chunks - 1) / chunks);
+    const int64_t chunks = std::min<int64_t>(
+        (n + 31) / 32, std::max<int64_t>(12, 32 * A.sm_count / targets));
+    P.W = (int)std::min<int64_t>(P.W, (n + chunks - 1) / chunks);
   }
   if (P.W < 1) return fail(TENEX_ERR_BADARG, "src_chunk must be >= 1");
   if (pairs) {

@@ -23,11 +23,10 @@ from tenex_b200.kernels import device as D
 # a whole SM's shared memory)
 TUNE_SPACE = [(0, 0, 512), (1024, 1, 512), (512, 2, 512), (512, 2, 256), (1024, 1, 256),
               (256, 4, 128), (256, 4, 256), (512, 2, 128), (1024, 1, 128), (256, 2, 64)]
-# Without autotuning the library picks the shape; 512 sources per item, fewer for few
-# genes. Measured
-# (ms per all-pairs launch): 10,000 x 20,000 (b_max 38) 989 vs 1097 for the old
-# 2 x 512 / 128 default; 5,000 x 10,000 (b_max 32) 256.0 vs 258.8; 2,000 x 5,000
-# (b_max 16) 11.37 vs 11.78 (11.14 for the best tuned shape).
+# Without autotuning the library picks the shape: its sources per item go with the gene
+# count. Default against the best shape of TUNE_SPACE, ms per all-pairs launch: 10,000 x
+# 20,000 (b_max 38) 635 / 635, 2,500 x 10,000 (b_max 32) 53.7 / 53.7, 2,000 x 5,000
+# (b_max 16) 7.15 / 7.11, 1,000 x 5,000 2.08 / 2.11.
 DEFAULT_CFG = dict(threads=0, ctas_per_sm=0, src_chunk=0)
 _tune_cache: dict[tuple, dict] = {}
 
