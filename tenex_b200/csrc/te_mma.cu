@@ -8,8 +8,8 @@
 // cell and sample where counting costs one shared-memory reduction per sample
 // (2.2e12 of them per second), so pairs of few cells come here (te_mma_layout) and the
 // others stay with te_pair.cu. Measured, all pairs, counting alone -> with this path:
-// 10,000 genes x 20,000 samples (b to 16, 5% to 38) 928 -> 662 ms, 2,000 x 5,000
-// (b to 16) 11.3 -> 7.8 ms, 3,281 x 458 (b to 7, every pair here) 7.1 -> 1.8 ms.
+// 10,000 genes x 20,000 samples (b to 16, 5% to 38) 873 -> 634 ms, 2,000 x 5,000
+// (b to 16) 10.6 -> 7.4 ms, 3,281 x 458 (b to 7, every pair here) 6.6 -> 1.7 ms.
 //
 //   * plan (one CTA): sources sorted by bin count and targets by occupied states are
 //     cut into tiles of at most 128 rows and 240 columns, whole genes only, so a
@@ -26,7 +26,9 @@
 //     and sample, not 4: 1.4 KB per 64 samples and tile instead of 12 KB, which L2
 //     could not deliver.
 //   * epilogue: a TMEM lane is one (source, y); it walks the columns of each target by
-//     xt, so c2b is a sum of its own registers. The terms are te_pair.cu's, operation
+//     xt, so c2b is a sum of its own registers. The xt that have columns come from one
+//     list of 8-byte words per half of the warps, without a loop over targets around
+//     them (3,281 x 458: 1.79 -> 1.66 ms, 2,000 x 5,000: 5.45 -> 5.36). The terms are te_pair.cu's, operation
 //     for operation; a lane's sum over a target's (or half a target's) columns is
 //     float32, as long a chain as te_pair.cu's, those over y are float64.
 //   * Bound: the shared-memory pipe (about 520 cycles per SM for a 256-sample step of a
@@ -65,6 +67,8 @@ constexpr int kTmemCols = 256;
 // kSplitCols columns or more (those of kSplitBins bins or more, which have at least
 // kSplitBins - 1 columns, are summed by two warps per lane quarter).
 constexpr int kSlots = 56, kSplitCols = 7, kSplitBins = 8;
+// xt with columns, and one without for a half of a target of kSplitBins bins that has none
+constexpr int kMaxGroups = kMaxCols + kSlots;
 constexpr int kBlkCache = 128;    // item blocks whose starts sit in shared memory
 static_assert(kSlots * kRows * 8 <= kStages * kStageBytes, "partial sums fit the stages");
 
@@ -545,6 +549,7 @@ __device__ __forceinline__ float group_sum(float acc, uint32_t taddr, int len, c
     uint32_t r[8];
     tmem_ld(taddr, r);
     switch (len) {
+      case 0: return acc;
       case 1: return group_terms<1>(acc, r, q, c1);
       case 2: return group_terms<2>(acc, r, q, c1);
       case 3: return group_terms<3>(acc, r, q, c1);
@@ -576,8 +581,12 @@ struct Tables {
   int wide0;             // first target of kSplitCols columns or more (targets ascend)
   float2 q[kMaxCols];    // M.colq
   int2 row[kMaxCols / 2];     // M.colrow of the columns this CTA expands
-  float c1[kSlots * 16];      // M.grp
-  uint8_t len[kSlots * 16];
+  // The xt of the tile's targets that have columns (M.grp), in the order in which the
+  // epilogue's two groups of warps take them: the first one's from the front on, the
+  // second one's from the back. {c1 (float), first column | columns << 8 | slot << 16 |
+  // last of its slot << 31}
+  uint2 grp[kMaxGroups];
+  int n_grp[2];
   int4 tgt[kSlots];      // M.tgt
   int src[kRows];             // genes of the sources
   uint8_t at[kRows + 1];      // their first rows in the tile; then the number of rows
@@ -648,10 +657,50 @@ __device__ void next_item(const TeMma& M, Shared& S, Tables& T, uint32_t* q_io, 
   }
   narrow = __reduce_add_sync(0xffffffffu, narrow);
   if (lane == 0) T.wide0 = narrow;
-  for (int k = lane; k < tt.y * 16; k += 32) {
-    const uint32_t g = M.grp[(int64_t)tt.x * 16 + k];
-    T.c1[k] = (float)(g & 0xffffffu);
-    T.len[k] = (uint8_t)(g >> 24);
+  // two targets at a time, a lane per xt
+  const int xt = lane & 15;
+  int n0 = 0, n1 = 0;
+#pragma unroll 2
+  for (int k = lane; k < (tt.y + 1) / 2 * 32; k += 32) {
+    const int t = k >> 4;
+    const bool in = t < tt.y;
+    const int4 v = in ? M.tgt[tt.x + t] : make_int4(0, 0, 0, 0);
+    const uint32_t g = xt < v.y ? M.grp[(int64_t)tt.x * 16 + k] : 0u;
+    const int len = (int)(g >> 24);
+    int at = len;  // columns up to and with this xt
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, at, o, 16);
+      if (xt >= o) at += below;
+    }
+    // targets of many bins: half of the xt each; the split depends on the target alone,
+    // so a pair's sum does not depend on its tile
+    const bool split = v.y >= kSplitBins;
+    const int mid = (v.y + (v.x & 1)) >> 1;
+    const int h = split ? xt >= mid : t & 1;
+    const uint32_t mine = lane < 16 ? 0xffffu : 0xffff0000u;  // this target's lanes
+    const uint32_t some0 = __ballot_sync(0xffffffffu, len > 0 && h == 0) & mine;
+    const uint32_t some1 = __ballot_sync(0xffffffffu, len > 0 && h == 1) & mine;
+    const uint32_t some = h ? some1 : some0;
+    const bool none = in && split && some == 0 && xt == (h ? mid : 0);
+    const bool put = len > 0 || none;
+    const uint32_t put0 = __ballot_sync(0xffffffffu, put && h == 0);
+    const uint32_t put1 = __ballot_sync(0xffffffffu, put && h == 1);
+    const uint32_t lt = (1u << lane) - 1;
+    const bool last = none || (some >> lane) == 1u;
+    if (put) {
+      const int i = h ? kMaxGroups - 1 - n1 - __popc(put1 & lt) : n0 + __popc(put0 & lt);
+      const int slot = (t < narrow ? t : 2 * t - narrow) + (split ? h : 0);
+      T.grp[i] = make_uint2(__float_as_uint((float)(g & 0xffffffu)),
+                            (uint32_t)(v.z - tt.z + at - len) | (uint32_t)len << 8 |
+                                (uint32_t)slot << 16 | (last ? 0x80000000u : 0u));
+    }
+    n0 += __popc(put0);
+    n1 += __popc(put1);
+  }
+  if (lane == 0) {
+    T.n_grp[0] = n0;
+    T.n_grp[1] = n1;
   }
   for (int s = lane; s < st.y; s += 32) {
     const int2 v = M.src[st.x + s];
@@ -702,12 +751,13 @@ __device__ void put_counts(const TeMma& M, const Tables& T, int tt, int row, uin
 
 // Two CTAs (a pair of SMs) share an item: 256 rows, each CTA's own 128 in its TMEM;
 // each expands half of the columns and the even one issues for both
-// (cta_group::2), so a column is expanded once per 256 rows. 10,000 x 20,000: 203 ms
-// (245 before the producers were split in two groups, the odd CTA's arrivals lost their
-// cluster-wide release and the epilogue its slow reciprocals and float64 sums), against
-// 315 ms with one CTA per 128-row tile. Row operands in TMEM instead of shared memory
-// (192 columns, three stages): 407 ms at a limit of 1,600 cells against 311 here; the
-// ring is then too short for its round trip of about 1,200 cycles.
+// (cta_group::2), so a column is expanded once per 256 rows. 10,000 x 20,000: 216 ms
+// for two thirds of the pairs. At one limit on cells: 203 ms, 245 before the producers
+// were split in two groups, the odd CTA's arrivals lost their cluster-wide release and
+// the epilogue its slow reciprocals and float64 sums, 315 with one CTA per 128-row tile.
+// Row operands in TMEM instead of shared memory (192 columns, three stages): 407 ms at a
+// limit of 1,600 cells against 311 here; the ring is then too short for its round trip of
+// about 1,200 cycles.
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_kernel(TeMma M) {
   if (*(volatile int*)&M.ws->bad_data != 0) return;
   const int n_items = M.ws->mma_items, n_blk = M.ws->mma_blocks, n_stiles = M.ws->mma_stiles;
@@ -874,34 +924,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
       const int half = warp >> 2, row = (warp & 3) * 32 + lane;
       const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
       if ((warp & 3) * 32 < n_rows) {
-        for (int tt = 0; tt < n_tgts; ++tt) {
-          const int4 t = T.tgt[tt];
-          const int c0 = t.z - T.tt.z, bt = t.y;
-          const int slot = tt < wide0 ? tt : 2 * tt - wide0;
-          // targets of many bins: half of the xt each; the split depends on the target
-          // alone, so a pair's sum does not depend on its tile
-          int j0 = 0, j1 = bt;
-          if (bt >= kSplitBins) {
-            const int mid = (bt + (t.x & 1)) >> 1;
-            j0 = half ? mid : 0;
-            j1 = half ? bt : mid;
-          } else if ((tt & 1) != half) {
-            j1 = 0;
+        const uint2* g = half ? T.grp + kMaxGroups - 1 : T.grp;
+        const int step = half ? -1 : 1, n = T.n_grp[half];
+        uint2 next = *g;
+        float sum = 0.f;
+        for (int i = 0; i < n; ++i) {
+          const float c1 = __uint_as_float(next.x);
+          const uint32_t w = next.y;
+          g += step;
+          if (i + 1 < n) next = *g;
+          const uint32_t at = w & 255u;
+          sum = group_sum(sum, lane_base + at, (int)(w >> 8 & 31u), T.q + at, c1);
+          if ((int32_t)w < 0) {
+            part[(w >> 16 & 127u) * kRows + row] = (double)sum;
+            sum = 0.f;
           }
-          if (j1 > 0) {
-            int at = c0;
-            for (int j = 0; j < j0; ++j) at += T.len[tt * 16 + j];
-            float sum = 0.f;
-            for (int j = j0; j < j1; ++j) {
-              const int len = T.len[tt * 16 + j];
-              if (len > 0)
-                sum = group_sum(sum, lane_base + (uint32_t)at, len, T.q + at, T.c1[tt * 16 + j]);
-              at += len;
-            }
-            part[(slot + (bt >= kSplitBins ? half : 0)) * kRows + row] = (double)sum;
-          }
-          if (M.counts_dbg != nullptr && half == 0) put_counts(M, T, tt, row, lane_base);
         }
+        if (M.counts_dbg != nullptr && half == 0)
+          for (int t = 0; t < n_tgts; ++t) put_counts(M, T, t, row, lane_base);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     } else {
@@ -994,10 +1034,11 @@ bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
   M->colrow = reinterpret_cast<int2*>(M->colq + cols);
   // A pair's cells (occupied target states x source bins) up to which the tensor cores
   // are the faster: their time goes with cells x samples, the counting kernel's with
-  // samples plus, per cell, its own entropy pass. Measured, ms of both kernels at a limit
-  // of 1,000 / 1,200 / 1,600 / 2,100 / 2,600 cells: 10,000 genes x 20,000 samples 665 /
-  // 662 / 671 / 694 / 725; 2,000 x 5,000 8.03 / 7.83 / 7.83 / 7.91 / 8.18; 2,000 x 600
-  // (b to 16) 4.82 / 4.66 / 4.19 / 3.93 / 3.76.
+  // samples plus, per cell, its own entropy pass. Measured, ms of both kernels with 900 /
+  // 1,050 / 1,200 / 1,400 for the 1,200 below: 10,000 genes x 20,000 samples 637 / 637 /
+  // 634 / 638; 2,000 x 5,000 7.10 / 7.14 / 7.22 / 7.34; 1,000 x 2,500 1.39 / 1.38 / 1.35 /
+  // 1.30; 301 x 101,003 2.35 / 2.17 / 2.12 / 2.21. Short series: 2,000 x 600 (b to 16) at
+  // a limit of 1,000 / 1,600 / 2,600 cells 4.82 / 4.19 / 3.76.
   const double N = M->N;
   M->max_cells = N <= 2078.0 ? 4096 : (int)(1200.0 * N / (N - 1470.0));
   M->cap_rows = std::min<int64_t>(rows, (int64_t)1 << 29);

@@ -1,4 +1,6 @@
-// te_pair.cu — persistent pair-tile transfer-entropy kernel for multi-bin data.
+// te_pair.cu — persistent pair-tile transfer-entropy kernel for multi-bin data, and the
+// launch driver of the TE entry points. All-pairs launches leave the pairs of few cells to
+// te_mma.cu (a source position below cut[target] is that kernel's).
 //
 // What it computes (reference: tenex/csrc/full_smem.cu:166-276 and
 // tenex/csrc/adaptive_smem.cu:158-273): for every ordered pair (source y ->
