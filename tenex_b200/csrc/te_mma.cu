@@ -28,9 +28,10 @@
 //   * epilogue: a TMEM lane is one (source, y); it walks the columns of each target by
 //     xt, so c2b is a sum of its own registers. The xt that have columns come from one
 //     list of 8-byte words per half of the warps, without a loop over targets around
-//     them (3,281 x 458: 1.79 -> 1.66 ms, 2,000 x 5,000: 5.45 -> 5.36). The terms are te_pair.cu's, operation
-//     for operation; a lane's sum over a target's (or half a target's) columns is
-//     float32, as long a chain as te_pair.cu's, those over y are float64.
+//     them (3,281 x 458: 1.79 -> 1.66 ms, 2,000 x 5,000: 5.45 -> 5.36). The terms are
+//     te_pair.cu's, operation for operation; a lane's sum over a target's (or half a
+//     target's) columns is float32, as long a chain as te_pair.cu's, those over y are
+//     float64.
 //   * Bound: the shared-memory pipe (about 520 cycles per SM for a 256-sample step of a
 //     256 x 240 tile: operands written, read by the MMAs, and the planes' loads; ncu: the
 //     load-store part of it 66% of the cycles, the tensor pipe 62%, the logic pipe 55%).

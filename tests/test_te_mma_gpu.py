@@ -118,3 +118,21 @@ def test_kernel_dimension_and_surrogate_statistics(cuda):
     assert torch.equal(acc[1], 2 * te.double() ** 2)
     assert torch.equal(cnt[off], 2 * (te >= obs).int()[off])
     assert not cnt[~off].any()
+
+
+@pytest.mark.parametrize("low", [0, 7, 13])
+def test_targets_that_use_few_of_their_bins(cuda, low):
+    """Targets of 16 bins whose values lie in three of them: one of the two halves that
+    the epilogue splits a target's bins into has no columns (low 0, 13) or both have."""
+    rng = np.random.default_rng(low)
+    n, T = 30, 700
+    bins = rng.integers(0, 3, (n, T)).astype(np.uint8)
+    npv = np.full(n, 3, np.int32)
+    bins[::2] += np.uint8(low)
+    npv[::2] = 16
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P = n * (n - 1)
+    te = [_run(db, npv_t, 16, 1, 0, P, cuda, tc).cpu().numpy() for tc in (True, False)]
+    assert np.max(np.abs(te[0] - O.te_pairfree(bins, npv, tau=1))) <= TOL
+    assert np.max(np.abs(te[0] - te[1])) <= TOL
