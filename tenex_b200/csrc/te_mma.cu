@@ -64,9 +64,10 @@ constexpr int kProducers = 256;   // threads that expand operands and run the ep
 constexpr int kThreads = kProducers + 32;
 constexpr uint32_t kSfCol = 248;  // TMEM columns of the unit scale factors
 constexpr int kTmemCols = 256;
-// Partial sums of a tile: one float64 row of kRows per target, two for targets of
-// kSplitCols columns or more (those of kSplitBins bins or more, which have at least
-// kSplitBins - 1 columns, are summed by two warps per lane quarter).
+// Partial sums of a tile: one float64 row (slot) of kRows per target, two for targets of
+// kSplitCols columns or more. Of the latter, those of kSplitBins bins or more are summed by
+// two warps per lane quarter, one per slot. Neither number implies the other: a target of 16
+// bins whose values lie in two of them, or whose series has few samples, has few columns.
 constexpr int kSlots = 56, kSplitCols = 7, kSplitBins = 8;
 // xt with columns, and one without for a half of a target of kSplitBins bins that has none
 constexpr int kMaxGroups = kMaxCols + kSlots;
@@ -674,9 +675,9 @@ __device__ void next_item(const TeMma& M, Shared& S, Tables& T, uint32_t* q_io, 
       const int below = __shfl_up_sync(0xffffffffu, at, o, 16);
       if (xt >= o) at += below;
     }
-    // targets of many bins: half of the xt each; the split depends on the target alone,
-    // so a pair's sum does not depend on its tile
-    const bool split = v.y >= kSplitBins;
+    // targets of many bins and with two slots: half of the xt each; the split depends on
+    // the target alone, so a pair's sum does not depend on its tile
+    const bool split = v.y >= kSplitBins && t >= narrow;
     const int mid = (v.y + (v.x & 1)) >> 1;
     const int h = split ? xt >= mid : t & 1;
     const uint32_t mine = lane < 16 ? 0xffffu : 0xffff0000u;  // this target's lanes
@@ -957,7 +958,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
       const double* a = part + (tt < wide0 ? tt : 2 * tt - wide0) * kRows;
       double tot = 0.0;
       const int y1 = T.at[s + 1];
-      if (t.y >= kSplitBins)
+      if (t.y >= kSplitBins && tt >= wide0)
         for (int y = T.at[s]; y < y1; ++y) tot += a[y] + a[y + kRows];
       else
         for (int y = T.at[s]; y < y1; ++y) tot += a[y];

@@ -136,3 +136,64 @@ def test_targets_that_use_few_of_their_bins(cuda, low):
     te = [_run(db, npv_t, 16, 1, 0, P, cuda, tc).cpu().numpy() for tc in (True, False)]
     assert np.max(np.abs(te[0] - O.te_pairfree(bins, npv, tau=1))) <= TOL
     assert np.max(np.abs(te[0] - te[1])) <= TOL
+
+
+def _all_outputs_match_oracle(bins, npv, bmax, lag, dev):
+    """Pair-free and matrix output and surrogate statistics of every pair, with the
+    tensor-core path, against the oracle. The value of N samples is a mean of N terms, so
+    TOL per sample holds for short series as for long ones."""
+    n = len(npv)
+    P, off = n * (n - 1), ~np.eye(n, dtype=bool)
+    db = D.pack_bins(bins, dev)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=dev)
+    ref = O.te_pairfree(bins, npv, tau=lag)
+    te = _run(db, npv_t, bmax, lag, 0, P, dev, True)
+    assert np.max(np.abs(te.cpu().numpy() - ref)) <= TOL
+    m = _run(db, npv_t, bmax, lag, 0, P, dev, True, matrix=True)
+    assert np.array_equal(m.cpu().numpy().T[off], te.cpu().numpy())
+    acc = [torch.zeros((n, n), dtype=torch.float64, device=dev) for _ in range(2)]
+    cnt = torch.zeros((n, n), dtype=torch.int32, device=dev)
+    D.surrogate_accumulate(db, npv_t, bmax, lag, m, acc[0], acc[1], cnt)
+    assert torch.equal(acc[0], m.double()) and torch.equal(acc[1], m.double() ** 2)
+    assert np.array_equal(cnt.cpu().numpy(), off.astype(np.int32))
+
+
+@pytest.mark.parametrize("wide", [0, 1, 6])
+def test_targets_of_many_bins_and_few_states(cuda, wide):
+    """Targets of 8 to 16 declared bins that use one or two of them (1 to 4 occupied
+    states): both low, both high, one of each half; beside each other in a tile and, with
+    `wide`, beside targets of many states."""
+    rng = np.random.default_rng(40 + wide)
+    T, rows, npv = 400, [], []
+    for b in (8, 9, 11, 16):
+        for v0, v1 in ((0, 0), (b - 1, b - 1), (0, 1), (b - 2, b - 1), (0, b - 1), (b // 2, 1)):
+            rows.append(np.where(rng.random(T) < 0.4, v0, v1))
+            npv.append(b)
+        rows.append(np.r_[np.zeros(T - 1, np.int64), b - 1])   # its second value comes last
+        npv.append(b)
+    for i in range(5 + wide):
+        b = 2 + i if i < 5 else 16
+        rows.append(rng.integers(0, b, T))
+        npv.append(b)
+    order = rng.permutation(len(rows))
+    bins = np.stack(rows)[order].astype(np.uint8)
+    _all_outputs_match_oracle(bins, np.array(npv, np.int32)[order], 16, 1, cuda)
+
+
+@pytest.mark.parametrize("T,lag", [(2, 1), (12, 6), (20, 15), (33, 31), (60, 50), (60, 53),
+                                   (300, 292)])
+def test_lag_close_to_the_length(cuda, T, lag):
+    """Dense genes of 8 to 16 bins with T - lag from 1 to 10: fewer samples than bins."""
+    bins, npv, bmax = _bins(1000 * T + lag, 70, T, 8, 16)
+    _all_outputs_match_oracle(bins[:, :, 0].astype(np.uint8), npv, bmax, lag, cuda)
+
+
+@pytest.mark.parametrize("T,tau", [(40, 39), (60, 54), (120, 111)])
+def test_engine_with_a_lag_close_to_the_length(cuda, T, tau):
+    from tenex_b200 import TransferEntropyEngine
+    rng = np.random.default_rng(T)
+    x = np.log1p(rng.poisson(3.0, (60, T)) * (rng.random((60, T)) < 0.7)).astype(np.float32)
+    res = TransferEntropyEngine(x, np.array([f"g{i}" for i in range(60)])).compute(
+        accelerator="gpu", tau=tau, kp=0.5)
+    ref = O.te_matrix(np.asarray(res.bin_arrs), np.asarray(res.n_per_var), tau=tau)
+    assert np.max(np.abs(res.matrix - ref)) <= TOL
