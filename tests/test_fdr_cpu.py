@@ -105,3 +105,31 @@ def test_blocked_cummin_equals_sequential(m):
     p = torch.rand(m, generator=g, dtype=torch.float64) ** 4
     ref = F.bh_adjust(p.numpy())
     assert np.allclose(bh_fdr_gpu(p, 0.05).numpy(), ref, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("fdr", [0.0, 1e-6, 0.01, 0.05, 0.5, 1.0, 1.5])
+@pytest.mark.parametrize("kind", ["ties", "spread", "one", "constant", "nan"])
+def test_threshold_keeps_the_edges_of_the_adjusted_p_values(fdr, kind):
+    """fdr_threshold_gpu keeps exactly the pairs whose Benjamini-Hochberg adjusted p-value
+    is below fdr, in their order, ties at the limit included."""
+    from tenex_b200.inference.fdr import fdr_threshold_gpu
+    from tenex_b200.inference.grn import bh_fdr_gpu
+    rng = np.random.default_rng(5)
+    te = rng.gamma(2.0, 0.02, 5000)
+    te[rng.random(5000) < 0.03] += 0.2 * rng.random()
+    if kind == "ties":
+        te = np.round(te, 2)
+    elif kind == "one":
+        te = te[:1]
+    elif kind == "constant":
+        te = np.full(50, 0.25)
+    elif kind == "nan":
+        te[17] = np.nan
+    te = torch.from_numpy(te.astype(np.float32))
+    pairs = torch.stack((torch.arange(len(te)), torch.arange(len(te)) + 1), 1)
+    got, got_pairs = fdr_threshold_gpu(te, pairs, fdr)
+    mask = torch.zeros(len(te), dtype=torch.bool)
+    if te.std() != 0:
+        z = (te - te.mean()) / te.std()
+        mask = bh_fdr_gpu(0.5 * torch.erfc(z / 1.4142135623730951), 0.05) < fdr
+    assert torch.equal(got, te[mask]) and torch.equal(got_pairs, pairs[mask])
