@@ -100,7 +100,7 @@ def to_device(a, device) -> torch.Tensor:
     if isinstance(a, torch.Tensor):
         if a.device.type == "cuda" or (torch.cuda.is_available() and a.is_pinned()):
             return a.to(device)             # already DMA-able: one direct copy
-        a = a.numpy()
+        a = a.detach().numpy()
     a = np.ascontiguousarray(a)
     device = torch.device(device)
     if device.type != "cuda" or a.nbytes < _DIRECT_BYTES or a.dtype == object:
