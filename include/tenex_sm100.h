@@ -87,9 +87,10 @@ size_t tenex_te_pairs_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 
 /* The same plus room for the tensor-core histograms of the all-pairs entry points:
  * tables (about 5 KB a gene) and bit planes (row_len / 4 bytes for each of a gene's
- * bins up to 16, at most 8 GiB). With a smaller workspace (256-byte aligned, at
- * least tenex_te_pairs_workspace_bytes) they use what fits, down to none: every
- * pair then runs in the shared-memory kernel. */
+ * bins up to 16, at most 8 GiB). With a smaller workspace (at least
+ * tenex_te_pairs_workspace_bytes) they use what fits, down to none: every pair then
+ * runs in the shared-memory kernel. The tables start at the workspace's next multiple
+ * of 256 bytes; an aligned workspace wastes none of it. */
 size_t tenex_te_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 
 /* The launch shape the histogram kernels would use on the current device for

@@ -1314,8 +1314,12 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   M.counts_dbg = counts;
   M.counts_stride = counts_stride;
   // pairs of few cells go to the tensor cores where the workspace has room for their
-  // tables and bit planes (one sized by tenex_te_workspace_bytes has)
-  if (!pairs && te_mma_layout(&M, wsb + ws_used, (int64_t)ws_bytes - ws_used)) P.cut = M.cut;
+  // tables and bit planes (one sized by tenex_te_workspace_bytes has), which hold 16-byte
+  // vectors and start at its next multiple of 256 bytes. The rest of the workspace holds
+  // whole words only, so callers may give it at any such address.
+  const int64_t skip = -(int64_t)(reinterpret_cast<uintptr_t>(wsb) + ws_used) & 255;
+  if (!pairs && te_mma_layout(&M, wsb + ws_used + skip, (int64_t)ws_bytes - ws_used - skip))
+    P.cut = M.cut;
   cudaError_t e = cudaMemsetAsync(workspace, 0, sizeof(WsHeader), stream);
   if (e != cudaSuccess) return check_cuda(e, "workspace reset");
   st = te_mma_launch(M, A, pairs != nullptr, stream);

@@ -197,3 +197,22 @@ def test_engine_with_a_lag_close_to_the_length(cuda, T, tau):
         accelerator="gpu", tau=tau, kp=0.5)
     ref = O.te_matrix(np.asarray(res.bin_arrs), np.asarray(res.n_per_var), tau=tau)
     assert np.max(np.abs(res.matrix - ref)) <= TOL
+
+
+@pytest.mark.parametrize("offset", [4, 8, 20, 128, 252])
+def test_workspace_at_any_word(cuda, offset):
+    """The entry points accept a workspace at any multiple of 4 bytes: the tensor-core
+    tables start at the next multiple of 256 bytes in it, in a smaller part of it."""
+    bins, npv, bmax = _bins(offset, 300, 900, 2, 16)
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P, s = 300 * 299, native.stream_ptr()
+    out = torch.zeros(P, dtype=torch.float32, device=cuda)
+    nb = D.workspace(cuda, 300, db.row_len, bmax).numel()
+    mem = torch.full((nb + 512,), 85, dtype=torch.uint8, device=cuda)
+    ws = mem[offset:offset + nb]
+    native.call("tenex_te_pairfree", db.ptr(), db.ld, npv_t.data_ptr(), bmax, 300, db.row_len, 1,
+                0, P, out.data_ptr(), native.OUT_PAIRFREE, 0, ws.data_ptr(), nb, None, s)
+    native.call("tenex_workspace_status", ws.data_ptr(), s)
+    assert np.max(np.abs(out.cpu().numpy() - O.te_pairfree(bins, npv, tau=1))) <= TOL
+    assert bool((mem[:offset] == 85).all()) and bool((mem[offset + nb:] == 85).all())
