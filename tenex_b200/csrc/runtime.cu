@@ -111,6 +111,7 @@ __global__ void block_shuffle_kernel(const uint8_t* __restrict__ in, int64_t in_
 // and merged at the block's end. 2,000 genes x 100 copies of 5,000 bytes (1 GB written):
 // 2.37 -> 1.09 ms; the kernel above gathers byte by byte from global memory.
 constexpr uint32_t kShufflePad = 32;  // zero bytes before and after the row
+constexpr int kShuffleSmem = 100 * 1024;  // most shared memory of a CTA: two share an SM
 __global__ void __launch_bounds__(256) block_shuffle_row_kernel(
     const uint8_t* __restrict__ in, int64_t in_ld, uint32_t row, uint32_t blK, uint32_t head,
     const int32_t* __restrict__ perm, int64_t perm_stride, int n_blocks, int copies, int per,
@@ -279,15 +280,17 @@ extern "C" int tenex_block_shuffle_many(const uint8_t* in, int64_t in_ld, int n_
   // several copies, rows that fit shared memory next to a second CTA, blocks of 16 bytes
   // or more (one copy: 10.8 us by the kernel above, 13.9 by this one, 1,000 x 5,000)
   const int64_t sh = row + 2 * kShufflePad;
-  if (n_copies > 1 && (int64_t)block_length * K >= 16 && sh <= 100 * 1024) {
+  if (n_copies > 1 && (int64_t)block_length * K >= 16 && sh <= kShuffleSmem) {
     DevAttr A;
     const int st = current_device_attr(&A);
     if (st) return st;
     // every copy in one CTA unless that leaves fewer than eight CTAs per SM
     const int groups = std::max(1, std::min(n_copies, 8 * A.sm_count / n_vars));
     const int per = (n_copies + groups - 1) / groups;
-    cudaError_t e = cudaFuncSetAttribute(block_shuffle_row_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    // always the same limit: it belongs to the function, and another thread's shorter
+    // rows must not lower it between this call and the launch
+    cudaError_t e = cudaFuncSetAttribute(
+        block_shuffle_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kShuffleSmem);
     if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute");
     block_shuffle_row_kernel<<<dim3((unsigned)n_vars, (unsigned)((n_copies + per - 1) / per)),
                                256, (size_t)sh, as_stream(stream)>>>(

@@ -229,3 +229,27 @@ def test_block_shuffles_bitexact_single_and_batched(cuda, T, K, bl):
         assert np.array_equal(got[s * n:(s + 1) * n], ref)
         one = D.block_shuffle(db, torch.as_tensor(perms[s], device=cuda), bl)
         assert np.array_equal(one.unpadded().cpu().numpy(), ref)
+
+
+def test_block_shuffles_of_several_lengths_from_threads(cuda):
+    """Rows of different lengths shuffled from several threads at once: the shared-memory
+    limit of the kernel is one per device, whatever a launch needs of it."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    def work(T):
+        rng = np.random.default_rng(T)
+        x = rng.integers(0, 9, (3, T)).astype(np.uint8)
+        nb = T // 20
+        perm = np.stack([[rng.permutation(nb) for _ in range(3)] for _ in range(2)])
+        with torch.cuda.stream(torch.cuda.Stream(cuda)):
+            db = D.pack_bins(x, cuda)
+            perm_t = torch.as_tensor(perm, dtype=torch.int32, device=cuda)
+            out = D.empty_bins(6, T, 1, cuda)
+            for _ in range(5000):
+                D.block_shuffle_many(db, perm_t, 20, out)
+            got = out.data[:, :T].cpu().numpy()
+        want = np.concatenate([O.block_shuffle(x, p, 20)[:, :, 0] for p in perm])
+        return bool(np.array_equal(got, want))
+
+    with ThreadPoolExecutor(max_workers=4) as ex:
+        assert all(ex.map(work, (1000, 90_000, 1500, 60_000)))
