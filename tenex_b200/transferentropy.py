@@ -29,8 +29,8 @@ import torch
 from tenex_b200 import _log
 from tenex_b200.kernels import compute_smem_bytes, query_smem_optin
 from tenex_b200.kernels import device as D
-from tenex_b200.kernels.adaptive_smem import compute_smem_bin_limit
-from tenex_b200.kernels.pair_tile import PairTileKernel
+from tenex_b200.kernels.adaptive_smem import AdaptiveSMEMKernel, compute_smem_bin_limit
+from tenex_b200.kernels.full_smem import FullSMEMKernel
 from tenex_b200.preprocess import compact_dtype, discretize
 from tenex_b200.result import TransferEntropyResult
 
@@ -268,8 +268,10 @@ class TransferEntropyEngine:
             return self._wrap_result()
 
         # prepare (coarsening) works on a copy so the cached bins stay intact; this
-        # package's kernels leave bins of at most the bin limit as they are
-        if isinstance(kobj, PairTileKernel) and b_max <= compute_smem_bin_limit(smem_optin):
+        # package's own kernels (not classes derived from them, which may have a prepare
+        # of their own) leave bins of at most the bin limit as they are
+        if (type(kobj) in (FullSMEMKernel, AdaptiveSMEMKernel)
+                and b_max <= compute_smem_bin_limit(smem_optin)):
             work, npv_w = db, npv
         else:
             work = D.DeviceBins(db.data.clone(), db.n, db.T, db.K)

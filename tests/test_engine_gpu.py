@@ -346,3 +346,28 @@ def test_staged_device_copy_back_equals_plain(cuda, dtype, shape):
     assert h.dtype == ref.dtype and h.shape == ref.shape and np.array_equal(h, ref)
     if t.dim() == 2:
         assert np.array_equal(D.to_host(t.t()), t.t().cpu().numpy())
+
+
+def test_derived_kernel_may_change_the_bins_in_prepare(cuda):
+    """A kernel class derived from this package's whose prepare works in place gets its
+    own copy of the bins: a second compute() on the cached bins gives the same result."""
+    from tenex_b200 import kernels as TK
+
+    class Halved(AdaptiveSMEMKernel):
+        name = "Halved"
+
+        def prepare(self, bin_arrs, n_per_var, b_max, **kwargs):
+            bin_arrs.data >>= 1
+            n_per_var.copy_((n_per_var + 1) // 2)
+            return bin_arrs, n_per_var, (b_max + 1) // 2
+
+    x, _ = W.cfg1_expression(n=30, T=300, seed=5, n_planted=2)
+    eng = TransferEntropyEngine(x, np.array([f"g{i}" for i in range(30)]))
+    TK.register(Halved())
+    try:
+        first = eng.compute(accelerator="gpu", kernel="Halved").matrix
+        again = eng.compute(accelerator="gpu", kernel="Halved")
+    finally:
+        TK._REGISTRY.pop()
+    assert np.array_equal(first, again.matrix)
+    assert np.max(np.abs(first - O.te_matrix(again.bin_arrs, again.n_per_var))) <= TOL
