@@ -385,6 +385,10 @@ int tenex_probe_tc_gemm_b2(int kind, int tile_n, int stages, double* ops, float*
  * of 8 independent chains (two min.f32 and one three-input max.f32 each); returns
  * the instruction count and the milliseconds. Synchronises `stream`. */
 int tenex_probe_minmax(int iters, double* instructions, float* ms, void* stream);
+/* Check (no reference counterpart): how many whole numbers c in [1, last], last <= 2^24,
+ * have an entropy-pass reciprocal other than the correctly rounded 1 / c in float32.
+ * Synchronises the stream. */
+int tenex_check_rcp_count(int64_t last, int64_t* differ, void* stream);
 
 #ifdef __cplusplus
 }

@@ -394,3 +394,38 @@ extern "C" int tenex_probe_minmax(int iters, double* instructions, float* ms, vo
   *instructions = (double)grid * block * iters * 8.0 * 3.0;
   return st;
 }
+
+namespace tenex {
+// dev::rcp_count against the correctly rounded reciprocal, one count per thread and step.
+__global__ void rcp_count_check(uint32_t last, unsigned* differ) {
+  unsigned n = 0;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x + 1; c <= last;
+       c += gridDim.x * blockDim.x)
+    n += __float_as_uint(dev::rcp_count((float)c)) != __float_as_uint(__frcp_rn((float)c));
+  if (n) atomicAdd(differ, n);
+}
+}  // namespace tenex
+
+extern "C" int tenex_check_rcp_count(int64_t last, int64_t* differ, void* stream_) {
+  if (last < 1 || last > ((int64_t)1 << 24) || !differ)
+    return fail(TENEX_ERR_BADARG, "need 1 <= last <= 2^24 and an output");
+  cudaStream_t s = as_stream(stream_);
+  unsigned* d = nullptr;
+  unsigned h = 0;
+  cudaError_t e = cudaMallocAsync(&d, sizeof(unsigned), s);
+  if (e != cudaSuccess) return check_cuda(e, "cudaMallocAsync");
+  e = cudaMemsetAsync(d, 0, sizeof(unsigned), s);
+  int st = e == cudaSuccess ? TENEX_OK : check_cuda(e, "cudaMemsetAsync");
+  if (!st) {
+    rcp_count_check<<<592, 256, 0, s>>>((uint32_t)last, d);
+    st = check_launch("rcp_count_check");
+  }
+  if (!st) {
+    e = cudaMemcpyAsync(&h, d, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) st = check_cuda(e, "tenex_check_rcp_count");
+  }
+  cudaFreeAsync(d, s);
+  *differ = h;
+  return st;
+}

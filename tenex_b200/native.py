@@ -113,6 +113,7 @@ _SIGS = {
                                ctypes.POINTER(ctypes.c_float), _P],
     "tenex_probe_minmax": [_I, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_float),
                            _P],
+    "tenex_check_rcp_count": [_L, ctypes.POINTER(ctypes.c_int64), _P],
 }
 _RESTYPES = {"tenex_te_workspace_bytes": ctypes.c_size_t,
              "tenex_te_pairs_workspace_bytes": ctypes.c_size_t,

@@ -387,3 +387,12 @@ def test_launch_shape_query(cuda):
     assert 0 < big["smem_bytes"] <= native.device_info(0).smem_optin
     with pytest.raises(native.TenexError):
         native.te_launch_shape(10, 10, 4)
+
+
+def test_count_reciprocal_is_correctly_rounded(cuda):
+    """The entropy passes' 1 / c equals the correctly rounded reciprocal for every count
+    that a float32 holds."""
+    import ctypes
+    differ = ctypes.c_int64(-1)
+    native.call("tenex_check_rcp_count", 1 << 24, ctypes.byref(differ), native.stream_ptr())
+    assert differ.value == 0
