@@ -371,3 +371,30 @@ def test_derived_kernel_may_change_the_bins_in_prepare(cuda):
         TK._REGISTRY.pop()
     assert np.array_equal(first, again.matrix)
     assert np.max(np.abs(first - O.te_matrix(again.bin_arrs, again.n_per_var))) <= TOL
+
+
+@pytest.mark.parametrize("n,m,tau", [(2, 1, 1), (2, 2, 2), (40, 40, 1), (300, 128, 1),
+                                     (300, 129, 3), (300, 257, 1)])
+def test_source_rows_match_oracle(cuda, n, m, tau):
+    """Source-filtered TE over one and several work items per target (128 sources each),
+    sources in any order; rows of other genes and the diagonal are 0."""
+    from tenex_b200.kernels.pair_list import te_source_rows
+    rng = np.random.default_rng(n + m)
+    bins, npv, bmax = O.remap(np.stack([rng.integers(0, b, 250) for b in
+                                        rng.integers(1, 9, n)]).astype(np.int32))
+    db = D.pack_bins(bins, cuda)
+    src = rng.permutation(n)[:m]
+    got = te_source_rows(db, torch.as_tensor(npv, dtype=torch.int32, device=cuda), bmax, tau,
+                         src).cpu().numpy()
+    want = np.zeros((n, n))
+    want[src] = O.te_matrix(bins, npv, tau=tau)[src]
+    assert np.max(np.abs(got - want)) <= TOL
+    assert not got.diagonal().any() and not np.delete(got, src, axis=0).any()
+
+
+def test_binarize_takes_a_tensor_that_requires_grad(cuda):
+    from tenex_b200.binarize import binarize
+    x = torch.linspace(-1, 1, 200).reshape(4, 50)
+    want = binarize(x, "mean", cuda)
+    got = binarize(x.requires_grad_(), "mean", cuda)
+    assert torch.equal(got[0].data, want[0].data) and torch.equal(got[3], want[3])
