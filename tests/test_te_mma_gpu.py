@@ -216,3 +216,24 @@ def test_workspace_at_any_word(cuda, offset):
     native.call("tenex_workspace_status", ws.data_ptr(), s)
     assert np.max(np.abs(out.cpu().numpy() - O.te_pairfree(bins, npv, tau=1))) <= TOL
     assert bool((mem[:offset] == 85).all()) and bool((mem[offset + nb:] == 85).all())
+
+
+@pytest.mark.parametrize("b_hi", [7, 16, 38])
+@pytest.mark.parametrize("part", [0.02, 0.3, 0.55, 0.9])
+def test_workspace_with_room_for_some_genes(cuda, b_hi, part):
+    """Between the least and the full workspace the bit planes reach only some of the
+    sources, cut inside a class of one bin count; the other pairs run in the
+    shared-memory kernel."""
+    bins, npv, bmax = _bins(b_hi, 300, 800, 2, b_hi)
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P, s = 300 * 299, native.stream_ptr()
+    out = torch.zeros(P, dtype=torch.float32, device=cuda)
+    full = D.workspace(cuda, 300, db.row_len, bmax).numel()
+    planes = 300 * min(bmax, 16) * (1024 // 8 * 2)          # the part that holds bit planes
+    nb = full - int(planes * (1 - part)) // 4 * 4
+    ws = torch.empty(nb, dtype=torch.uint8, device=cuda)
+    native.call("tenex_te_pairfree", db.ptr(), db.ld, npv_t.data_ptr(), bmax, 300, db.row_len, 1,
+                0, P, out.data_ptr(), native.OUT_PAIRFREE, 0, ws.data_ptr(), nb, None, s)
+    native.call("tenex_workspace_status", ws.data_ptr(), s)
+    assert np.max(np.abs(out.cpu().numpy() - O.te_pairfree(bins, npv, tau=1))) <= TOL
