@@ -369,8 +369,8 @@ __global__ void __launch_bounds__(1024) plan_kernel(TeMma M) {
       cols += S.width[S.cls[i]];
       widest = S.cls[i];
     }
-    const int fair = (int)((int64_t)cols * ((n_stiles + 1) / 2) / M.sm_pairs);
-    S.room = min(kMaxCols, max(max(64, widest), (fair + 15) & ~15));
+    const int64_t fair = (int64_t)cols * ((n_stiles + 1) / 2) / M.sm_pairs;
+    S.room = min(kMaxCols, max(max(64, widest), ((int)min(fair, (int64_t)kMaxCols) + 15) & ~15));
   }
   __syncthreads();
   pack_tiles(S, 1, kMaxCols, S.room, kSlots, kSplitCols, n, tid);
@@ -1008,6 +1008,11 @@ bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
   M->cap_rows = 0;
   if (M->row_len >= ((int64_t)1 << 24)) return false;
   const int n = M->n;
+  // work items are counted in 32 bits: at most one per target and pair of source tiles (a
+  // full tile has over kRows - bins rows). Beyond 170,000 genes of 16 bins.
+  const int64_t c = std::min(M->b_max, kMaxSrcBins);
+  const int64_t tile_pairs = ((int64_t)n * c / (kRows + 1 - c) + 2) / 2;
+  if ((int64_t)(M->t_last - M->t_first + 1) * tile_pairs > 0x7fffffff) return false;
   M->words = (int)(round_up(M->row_len, 256) / 32);
   const int64_t cols = col_bound(n, M->b_max);
   const int64_t fixed = tables_bytes(n) + round_up(cols * 16, 256) + 256;
