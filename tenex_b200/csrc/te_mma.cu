@@ -28,10 +28,14 @@
 //   * epilogue: a TMEM lane is one (source, y); it walks the columns of each target by
 //     xt, so c2b is a sum of its own registers. The xt that have columns come from one
 //     list of 8-byte words per half of the warps, without a loop over targets around
-//     them (3,281 x 458: 1.79 -> 1.66 ms, 2,000 x 5,000: 5.45 -> 5.36). The terms are
-//     te_pair.cu's, operation for operation; a lane's sum over a target's (or half a
-//     target's) columns is float32, as long a chain as te_pair.cu's, those over y are
-//     float64.
+//     them (the kernel alone, 3,281 x 458: 1.79 -> 1.66 ms, 2,000 x 5,000: 5.45 -> 5.36).
+//     The terms are te_pair.cu's, operation for operation. Those of one xt, 16 at most,
+//     are added in float32, their sums over xt and y in float64, so no chain is longer
+//     than te_pair.cu's. One float32 chain over a target's columns (up to 240 terms)
+//     left 300 samples of 15 bins against 3 up to 2.4 times (root mean square 1.4 times)
+//     as far from the float64 oracle as te_pair.cu does; float64 costs, whole launch,
+//     3,281 x 458 1.75 -> 1.81 ms, 2,000 x 5,000 7.39 -> 7.49, 10,000 x 20,000 634.5 ->
+//     636.0 (a compensated float32 sum: 1.85, 7.52, 636.3).
 //   * Bound: the shared-memory pipe (about 520 cycles per SM for a 256-sample step of a
 //     256 x 240 tile: operands written, read by the MMAs, and the planes' loads; ncu: the
 //     load-store part of it 66% of the cycles, the tensor pipe 62%, the logic pipe 55%).
@@ -929,17 +933,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
         const uint2* g = half ? T.grp + kMaxGroups - 1 : T.grp;
         const int step = half ? -1 : 1, n = T.n_grp[half];
         uint2 next = *g;
-        float sum = 0.f;
+        double sum = 0.0;
         for (int i = 0; i < n; ++i) {
           const float c1 = __uint_as_float(next.x);
           const uint32_t w = next.y;
           g += step;
           if (i + 1 < n) next = *g;
           const uint32_t at = w & 255u;
-          sum = group_sum(sum, lane_base + at, (int)(w >> 8 & 31u), T.q + at, c1);
+          sum += (double)group_sum(0.f, lane_base + at, (int)(w >> 8 & 31u), T.q + at, c1);
           if ((int32_t)w < 0) {
-            part[(w >> 16 & 127u) * kRows + row] = (double)sum;
-            sum = 0.f;
+            part[(w >> 16 & 127u) * kRows + row] = sum;
+            sum = 0.0;
           }
         }
         if (M.counts_dbg != nullptr && half == 0)

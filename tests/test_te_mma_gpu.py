@@ -237,3 +237,25 @@ def test_workspace_with_room_for_some_genes(cuda, b_hi, part):
                 0, P, out.data_ptr(), native.OUT_PAIRFREE, 0, ws.data_ptr(), nb, None, s)
     native.call("tenex_workspace_status", ws.data_ptr(), s)
     assert np.max(np.abs(out.cpu().numpy() - O.te_pairfree(bins, npv, tau=1))) <= TOL
+
+
+@pytest.mark.parametrize("bt,bs", [(15, 3), (13, 8), (7, 2)])
+def test_error_is_no_larger_than_the_counting_kernels(cuda, bt, bs):
+    """Root mean square error against the float64 oracle on short series, where TE and so
+    the sums are large. Both kernels add float32 terms in chains of a column or so and the
+    rest in float64, so their errors have one size; 10% is left for the 1% by which the
+    root mean square of 19,600 errors varies and the terms' order."""
+    n, T = 280, 300
+    rng = np.random.default_rng(bt)
+    bins, npv, bmax = O.remap(np.stack(
+        [rng.integers(0, bt if i % 2 else bs, T) for i in range(n)]).astype(np.int32))
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P = n * (n - 1)
+    ids = np.arange(P)
+    tgt, src = ids // (n - 1), ids % (n - 1)
+    mine = (npv[tgt] == bt) & (npv[src + (src >= tgt)] == bs)
+    ref = O.te_pairfree(bins, npv, tau=1)
+    rms = [float(np.sqrt(np.mean((_run(db, npv_t, bmax, 1, 0, P, cuda, tc).cpu().numpy().astype(
+        np.float64) - ref)[mine] ** 2))) for tc in (True, False)]
+    assert mine.sum() == 140 * 140 and rms[0] <= 1.1 * rms[1]
