@@ -360,7 +360,11 @@ __host__ __device__ inline bool in_smem(int64_t bt, int64_t bs, int N, int mbmax
 // rounding residue). Empty cells add 0 times a finite logarithm (no branch).
 // A column's terms are added in float32, the columns in float64: how many columns a lane
 // has goes with the group's size, and one float32 chain over all of them was up to 1.3
-// times as far off for groups of fewer warps (700 samples, 16 bins against 3).
+// times as far off for groups of fewer warps (700 samples, 16 bins against 3). te_mma.cu
+// adds the same way, so a pair's value depends neither on the launch shape, the pair range
+// or the counter width nor on which kernel counts it (but for the last bit of a float64
+// sum, too little to change its float32 rounding in 4 million pairs): a surrogate whose
+// counts equal the observed ones ties with the observed TE, whatever made either.
 template <bool PACK16, bool CLEAR>
 __device__ __forceinline__ double entropy_cols(uint32_t* tab, int bt, int bs, int stride,
                                               const int* c1i, const float2* qa, int lane_g,
@@ -381,6 +385,7 @@ __device__ __forceinline__ double entropy_cols(uint32_t* tab, int bt, int bs, in
     const float2* q = qa + j;  // {c1/c2a, c2a}
     float acc = 0.f;
     if (PACK16) {
+      float odd = 0.f;
       const float blo = (float)(s & 0xffffu), bhi = (float)(s >> 16);
       const float inv_lo = dev::rcp_count(fmaxf(blo, 1.f));
       const float inv_hi = dev::rcp_count(fmaxf(bhi, 1.f));
@@ -389,8 +394,9 @@ __device__ __forceinline__ double entropy_cols(uint32_t* tab, int bt, int bs, in
         const uint32_t w = *p;
         if (CLEAR) *p = 0u;
         acc = dev::add_term(acc, (float)(w & 0xffffu), c1j, blo, inv_lo, *q);
-        acc = dev::add_term(acc, (float)(w >> 16), c1j, bhi, inv_hi, *q);
+        odd = dev::add_term(odd, (float)(w >> 16), c1j, bhi, inv_hi, *q);
       }
+      sum += (double)odd;
     } else {
       const float b = (float)s;
       const float inv = dev::rcp_count(b);

@@ -259,3 +259,29 @@ def test_error_is_no_larger_than_the_counting_kernels(cuda, bt, bs):
     rms = [float(np.sqrt(np.mean((_run(db, npv_t, bmax, 1, 0, P, cuda, tc).cpu().numpy().astype(
         np.float64) - ref)[mine] ** 2))) for tc in (True, False)]
     assert mine.sum() == 140 * 140 and rms[0] <= 1.1 * rms[1]
+
+
+@pytest.mark.parametrize("n,T,b", [(260, 300, (2, 16)), (300, 1200, (2, 12)),
+                                   (250, 2000, (2, 38)), (230, 70000, (2, 24))])
+def test_value_of_a_pair_is_the_same_by_every_route(cuda, n, T, b):
+    """Tensor cores or shared-memory counters of 32 or 16 bits, any launch shape, pair range
+    or list: the terms of a column are added in one order in float32, all else in
+    float64, whose order leaves a float32 result of these inputs alone."""
+    from tenex_b200.kernels.pair_list import te_pair_list
+    bins, npv, bmax = _bins(n + T, n, T, *b, skew=True)
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P = n * (n - 1)
+    te = _run(db, npv_t, bmax, 1, 0, P, cuda, True)
+    assert torch.equal(te, _run(db, npv_t, bmax, 1, 0, P, cuda, False))
+    for p0, cnt in ((0, 50), (P // 2 - 7, 3 * n), (P - n, n)):
+        for tc in (True, False):
+            assert torch.equal(te[p0:p0 + cnt], _run(db, npv_t, bmax, 1, p0, cnt, cuda, tc))
+    for cfg in (dict(threads=1024, ctas_per_sm=1, src_chunk=512),
+                dict(threads=256, ctas_per_sm=2, src_chunk=64),
+                dict(threads=128, ctas_per_sm=4, src_chunk=7)):
+        assert torch.equal(te, D.te_pairfree(db, npv_t, bmax, 1, cfg=cfg))
+    ids = np.random.default_rng(n).integers(0, P, 2000)
+    tgt, loc = ids // (n - 1), ids % (n - 1)
+    pl = te_pair_list(db, npv_t, bmax, 1, np.stack((tgt, loc + (loc >= tgt)), 1))
+    assert torch.equal(te[torch.as_tensor(ids, device=cuda)], pl)
