@@ -100,6 +100,20 @@ __device__ __forceinline__ float add_term(float acc, float c, float c1, float c2
   return acc;
 }
 
+// Sums of terms in whole multiples of 2^-32, whose order does not matter: of counts below
+// 2^24 the terms' absolute sum is below 2^29, so 64 bits hold it. x is a float32 sum of few
+// terms; what the conversion drops is below 2^-32.
+constexpr double kFixedOne = 4294967296.0;
+__device__ __forceinline__ long long to_fixed(float x) {
+  return __float2ll_rn(x * (float)kFixedOne);
+}
+
+__device__ __forceinline__ long long warp_sum(long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Named barrier over `nthreads` threads (a multiple of 32) with id in [1, 15].
 __device__ __forceinline__ void named_bar(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

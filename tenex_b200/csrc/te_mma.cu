@@ -30,12 +30,13 @@
 //     list of 8-byte words per half of the warps, without a loop over targets around
 //     them (the kernel alone, 3,281 x 458: 1.79 -> 1.66 ms, 2,000 x 5,000: 5.45 -> 5.36).
 //     The terms are te_pair.cu's, operation for operation. Those of one xt, 16 at most,
-//     are added in float32, their sums over xt and y in float64, so no chain is longer
-//     than te_pair.cu's. One float32 chain over a target's columns (up to 240 terms)
-//     left 300 samples of 15 bins against 3 up to 2.4 times (root mean square 1.4 times)
-//     as far from the float64 oracle as te_pair.cu does; float64 costs, whole launch,
-//     3,281 x 458 1.75 -> 1.81 ms, 2,000 x 5,000 7.39 -> 7.49, 10,000 x 20,000 634.5 ->
-//     636.0 (a compensated float32 sum: 1.85, 7.52, 636.3).
+//     are added in float32, their sums over xt and y in 2^-32 fixed point, so no chain is
+//     longer than te_pair.cu's and every order gives the same bits. One float32 chain over
+//     a target's columns (up to 240 terms) left 300 samples of 15 bins against 3 up to 2.4
+//     times (root mean square 1.4 times) as far from the float64 oracle as te_pair.cu does.
+//     Whole launch with that chain / float64 / fixed point: 3,281 x 458 1.75 / 1.81 / 1.78
+//     ms, 2,000 x 5,000 7.39 / 7.48 / 7.37, 10,000 x 20,000 634.5 / 636 / 632.8 (a
+//     compensated float32 sum: 1.85, 7.52, 636.3).
 //   * Bound: the shared-memory pipe (about 520 cycles per SM for a 256-sample step of a
 //     256 x 240 tile: operands written, read by the MMAs, and the planes' loads; ncu: the
 //     load-store part of it 66% of the cycles, the tensor pipe 62%, the logic pipe 55%).
@@ -68,7 +69,7 @@ constexpr int kProducers = 256;   // threads that expand operands and run the ep
 constexpr int kThreads = kProducers + 32;
 constexpr uint32_t kSfCol = 248;  // TMEM columns of the unit scale factors
 constexpr int kTmemCols = 256;
-// Partial sums of a tile: one float64 row (slot) of kRows per target, two for targets of
+// Partial sums of a tile: one row (slot) of kRows 64-bit sums per target, two for targets of
 // kSplitCols columns or more. Of the latter, those of kSplitBins bins or more are summed by
 // two warps per lane quarter, one per slot. Neither number implies the other: a target of 16
 // bins whose values lie in two of them, or whose series has few samples, has few columns.
@@ -716,10 +717,10 @@ __device__ void next_item(const TeMma& M, Shared& S, Tables& T, uint32_t* q_io, 
 }
 
 // One pair's TE to the launch's output (one thread per pair).
-__device__ __forceinline__ void put_pair(const TeMma& M, int src, int tgt, double tot) {
+__device__ __forceinline__ void put_pair(const TeMma& M, int src, int tgt, long long tot) {
   const int64_t p = (int64_t)tgt * (M.n - 1) + (src < tgt ? src : src - 1);
   if (src == tgt || p < M.p0 || p >= M.p1) return;
-  const float te = (float)(tot * M.inv_N);
+  const float te = (float)((double)tot * M.inv_unit);
   if (M.out_mode == kOutPairfree) {
     M.out[p - M.p0] = te;
   } else if (M.out_mode == kOutMatrix) {
@@ -771,7 +772,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* stages = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Shared& S = *reinterpret_cast<Shared*>(stages + kStages * kStageBytes);
-  double* part = reinterpret_cast<double*>(stages);  // [slot][row], epilogue only
+  long long* part = reinterpret_cast<long long*>(stages);  // [slot][row], epilogue only
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_rank();
   const int n_steps = (M.N + 255) >> 8;
@@ -933,17 +934,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
         const uint2* g = half ? T.grp + kMaxGroups - 1 : T.grp;
         const int step = half ? -1 : 1, n = T.n_grp[half];
         uint2 next = *g;
-        double sum = 0.0;
+        long long sum = 0;
         for (int i = 0; i < n; ++i) {
           const float c1 = __uint_as_float(next.x);
           const uint32_t w = next.y;
           g += step;
           if (i + 1 < n) next = *g;
           const uint32_t at = w & 255u;
-          sum += (double)group_sum(0.f, lane_base + at, (int)(w >> 8 & 31u), T.q + at, c1);
+          sum += dev::to_fixed(group_sum(0.f, lane_base + at, (int)(w >> 8 & 31u), T.q + at, c1));
           if ((int32_t)w < 0) {
             part[(w >> 16 & 127u) * kRows + row] = sum;
-            sum = 0.0;
+            sum = 0;
           }
         }
         if (M.counts_dbg != nullptr && half == 0)
@@ -959,8 +960,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
       const int tt = i / n_src, s = i - tt * n_src;
       const int4 t = T.tgt[tt];
       if (T.st.x + s >= t.w) continue;  // te_pair.cu's pair
-      const double* a = part + (tt < wide0 ? tt : 2 * tt - wide0) * kRows;
-      double tot = 0.0;
+      const long long* a = part + (tt < wide0 ? tt : 2 * tt - wide0) * kRows;
+      long long tot = 0;
       const int y1 = T.at[s + 1];
       if (t.y >= kSplitBins && tt >= wide0)
         for (int y = T.at[s]; y < y1; ++y) tot += a[y] + a[y + kRows];

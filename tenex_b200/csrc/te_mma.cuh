@@ -17,7 +17,7 @@ struct TeMma {
   int64_t ld;
   const int32_t* npv;
   int n, N, lag, b_max;
-  double inv_N;
+  double inv_unit;   // 1 / N, divided by to_fixed's 2^32
   int64_t row_len;
   int64_t p0, p1;
   int t_first, t_last;

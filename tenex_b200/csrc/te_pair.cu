@@ -59,6 +59,7 @@ struct TeParams {
   const int32_t* npv;
   int n;
   int N;          // samples per pair (row_len - lag), < 2^31
+  double inv_unit; // 1 / N, divided by to_fixed's 2^32 unless big
   int lag;
   int ztile;      // samples of the target staged at a time (N: the whole series)
   int big;        // N >= 2^24: float64 entropy pass
@@ -358,18 +359,19 @@ __host__ __device__ inline bool in_smem(int64_t bt, int64_t bs, int N, int mbmax
 // except where c3 * c1 == c2a * c2b, whose term is exactly 0 as in the
 // reference's formula (constant or duplicated sources give TE = 0, not a
 // rounding residue). Empty cells add 0 times a finite logarithm (no branch).
-// A column's terms are added in float32, the columns in float64: how many columns a lane
-// has goes with the group's size, and one float32 chain over all of them was up to 1.3
-// times as far off for groups of fewer warps (700 samples, 16 bins against 3). te_mma.cu
-// adds the same way, so a pair's value depends neither on the launch shape, the pair range
-// or the counter width nor on which kernel counts it (but for the last bit of a float64
-// sum, too little to change its float32 rounding in 4 million pairs): a surrogate whose
+// A column's terms are added in float32, the columns in 2^-32 fixed point: how many
+// columns a lane has goes with the group's size, and one float32 chain over all of them
+// was up to 1.3 times as far off for groups of fewer warps (700 samples, 16 bins against
+// 3). te_mma.cu adds the same way, so a pair's value depends neither on the launch shape,
+// the pair range or the counter width nor on which kernel counts it: a surrogate whose
 // counts equal the observed ones ties with the observed TE, whatever made either.
+// 2,500 x 10,000 (b to 32) 52.9 ms with the float32 chain, 53.5 so (float64: 53.1, equal
+// but for one pair in some millions).
 template <bool PACK16, bool CLEAR>
-__device__ __forceinline__ double entropy_cols(uint32_t* tab, int bt, int bs, int stride,
+__device__ __forceinline__ long long entropy_cols(uint32_t* tab, int bt, int bs, int stride,
                                               const int* c1i, const float2* qa, int lane_g,
                                               int gthreads) {
-  double sum = 0.0;
+  long long sum = 0;
   // every word of a row, padding included (zero, so skipped by the s == 0 test):
   // consecutive lanes then read consecutive words, one wavefront per warp
   const int ncy = stride;
@@ -396,7 +398,7 @@ __device__ __forceinline__ double entropy_cols(uint32_t* tab, int bt, int bs, in
         acc = dev::add_term(acc, (float)(w & 0xffffu), c1j, blo, inv_lo, *q);
         odd = dev::add_term(odd, (float)(w >> 16), c1j, bhi, inv_hi, *q);
       }
-      sum += (double)odd;
+      sum += dev::to_fixed(odd);
     } else {
       const float b = (float)s;
       const float inv = dev::rcp_count(b);
@@ -407,7 +409,7 @@ __device__ __forceinline__ double entropy_cols(uint32_t* tab, int bt, int bs, in
         acc = dev::add_term(acc, (float)w, c1j, b, inv, *q);
       }
     }
-    sum += (double)acc;
+    sum += dev::to_fixed(acc);
   }
   return sum;
 }
@@ -449,7 +451,7 @@ struct ItemCtx {
   const int* c1i;
   const int* c2ai;
   const float2* qa;
-  double* red;
+  long long* red;
   int slot_region;    // shared-memory slot region (overflow split rule)
   bool pad;           // table rows at an odd stride (row words | 1)
   const uint2* zperm; // sorted 16-sample groups of 1-byte states, or nullptr
@@ -496,10 +498,10 @@ __device__ __forceinline__ bool pair_of(const TeParams& P, const ItemCtx& it, in
 // (same expression and exact-zero rule as the cell pass) are summed in 2^-32 fixed
 // point, so the total does not depend on which sample claimed a cell or on the
 // order of the additions: bitwise reproducible. Returns the CTA's total.
-__device__ double entropy_samples_gmem(uint32_t* tab, uint32_t* c2b, const unsigned char* zsm,
+__device__ long long entropy_samples_gmem(uint32_t* tab, uint32_t* c2b, const unsigned char* zsm,
                                        bool z8, const uint8_t* srow, int N, int bt, int bs,
                                        const int* c1i, const float2* qa, int tid, int nthreads,
-                                       double* red) {
+                                       long long* red) {
   const uint16_t* z16 = reinterpret_cast<const uint16_t*>(zsm);
   for (int s = tid; s < N; s += nthreads) {
     const uint32_t z = z8 ? zsm[s] : z16[s];
@@ -520,18 +522,17 @@ __device__ double entropy_samples_gmem(uint32_t* tab, uint32_t* c2b, const unsig
     const bool e = cf * (float)c1i[x0] == q.y * b;
     const float r = e ? 1.f : cf * __frcp_rn(b) * q.x;
     const float term = cf * __log2f(r);
-    acc += __float2ll_rn(term * 4294967296.0f);  // |term| * 2^32 < 2^63 for N < 2^24
+    acc += dev::to_fixed(term);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  long long* red64 = reinterpret_cast<long long*>(red);
-  if ((tid & 31) == 0) red64[tid >> 5] = acc;
+  if ((tid & 31) == 0) red[tid >> 5] = acc;
   __syncthreads();
   long long tot = 0;
-  for (int w = 0; w < (nthreads >> 5); ++w) tot += red64[w];
+  for (int w = 0; w < (nthreads >> 5); ++w) tot += red[w];
   // c2b back to zero for the next pair (b_t * b_s words)
   for (int i = tid; i < bt * bs; i += nthreads) c2b[i] = 0u;
   __syncthreads();
-  return (double)tot * (1.0 / 4294967296.0);
+  return tot;
 }
 
 // After the histogram of source src (pair id p) is complete in the group's
@@ -562,7 +563,8 @@ __device__ __forceinline__ void finish_pair(const TeParams& P, const ItemCtx& it
   }
 
   // -- entropy pass (shared slots are cleared for the next source) ---------
-  double tot;
+  // the pair's sum in to_fixed's unit; series of 2^24 samples or more: a float64's bits
+  long long tot;
   bool cta_total = false;  // tot already holds the whole CTA's sum
   if (MODE == kGmem && P.gc2b != nullptr && !P.big && P.ztile >= P.N) {
     tot = entropy_samples_gmem(tab, P.gc2b + (int64_t)blockIdx.x * P.gc2b_words, it.zsm, it.z8,
@@ -570,8 +572,8 @@ __device__ __forceinline__ void finish_pair(const TeParams& P, const ItemCtx& it
                                G * 32, it.red);
     cta_total = true;
   } else if (P.big) {
-    tot = dev::warp_sum(entropy_cols_f64<true>(tab, bt, bs, stride, it.c1i, it.c2ai, lane_g,
-                                                gthreads));
+    tot = __double_as_longlong(dev::warp_sum(
+        entropy_cols_f64<true>(tab, bt, bs, stride, it.c1i, it.c2ai, lane_g, gthreads)));
   } else {
     tot = dev::warp_sum(
         entropy_cols<PACK16, true>(tab, bt, bs, stride, it.c1i, it.qa, lane_g, gthreads));
@@ -580,12 +582,15 @@ __device__ __forceinline__ void finish_pair(const TeParams& P, const ItemCtx& it
     if ((tid & 31) == 0) it.red[warp] = tot;
     dev::named_bar(1 + g, gthreads);
     if (lane_g == 0) {
-      tot = 0.0;
-      for (int w = 0; w < G; ++w) tot += it.red[g * G + w];
+      const long long* r = it.red + g * G;
+      tot = r[0];
+      for (int w = 1; w < G; ++w)
+        tot = P.big ? __double_as_longlong(__longlong_as_double(tot) + __longlong_as_double(r[w]))
+                    : tot + r[w];
     }
   }
   if (lane_g == 0) {
-    const float te = (float)(tot / (double)P.N);
+    const float te = (float)((P.big ? __longlong_as_double(tot) : (double)tot) * P.inv_unit);
     if (P.out_mode == kOutPairfree) {
       P.out[p - P.p0] = te;
     } else if (P.out_mode == kOutMatrix) {
@@ -734,7 +739,7 @@ __global__ void __launch_bounds__(1024, 1) te_pair_tile_kernel(TeParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemLayout SL = smem_layout(P.ztile, P.zbytes, P.bmax, P.mbmax);
   int* misc = reinterpret_cast<int*>(smem + SL.misc_off);
-  double* red = reinterpret_cast<double*>(smem + SL.red_off);
+  long long* red = reinterpret_cast<long long*>(smem + SL.red_off);
   int* c1i = reinterpret_cast<int*>(smem + SL.c1_off);
   int* const c2a_sm = reinterpret_cast<int*>(smem + SL.c2a_off);
   float2* const qa_sm = reinterpret_cast<float2*>(smem + SL.q_off);
@@ -1246,6 +1251,7 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   P.ztile = z_tile(P.N, P.zbytes);
   P.mbmax = marginal_bound(b_max, P.ztile, P.zbytes, smem_one_cta(A));
   P.big = P.N >= (1 << 24) ? 1 : 0;
+  P.inv_unit = 1.0 / (P.big ? (double)P.N : P.N * dev::kFixedOne);
   P.out_mode = out_mode;
   P.out = out;
   P.out_ld = out_ld;
@@ -1304,7 +1310,7 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   M.npv = npv;
   M.n = n;
   M.N = P.N;
-  M.inv_N = 1.0 / (double)P.N;
+  M.inv_unit = P.inv_unit;
   M.lag = P.lag;
   M.b_max = b_max;
   M.row_len = row_len;
