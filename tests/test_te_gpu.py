@@ -396,3 +396,14 @@ def test_count_reciprocal_is_correctly_rounded(cuda):
     differ = ctypes.c_int64(-1)
     native.call("tenex_check_rcp_count", 1 << 24, ctypes.byref(differ), native.stream_ptr())
     assert differ.value == 0
+
+
+@pytest.mark.parametrize("n", [2, 3, 8, 14, 23, 24, 25])
+@pytest.mark.parametrize("b,T", [(13, 400), (13, 70_001), (15, 70_001), (24, 900), (30, 70_001)])
+def test_items_of_few_sources(cuda, n, b, T):
+    """Work items whose sources are around once and twice the histogram slots of a CTA
+    (3 to 15 here): warps per source chosen by rounds; whole and tiled series."""
+    rng = np.random.default_rng(n * b)
+    bins, npv, bmax = O.remap(rng.integers(0, b, (n, T)).astype(np.int32))
+    te = _gpu_te(bins, npv, bmax, cuda).cpu().numpy()
+    assert np.max(np.abs(te - O.te_pairfree(bins, npv))) <= TOL
