@@ -85,9 +85,9 @@ int tenex_device_query(int device, tenex_dev_info* info);
  * makes such a call fail with the size it needs. */
 size_t tenex_te_pairs_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 
-/* The same plus room for the tensor-core histograms of the all-pairs entry points:
- * tables (about 5 KB a gene) and bit planes (row_len / 4 bytes for each of a gene's
- * bins up to 16, at most 8 GiB). With a smaller workspace (at least
+/* The same plus room for the tensor-core histograms of the all-pairs entry points, where
+ * all pairs of n_vars genes are enough work for them: tables (about 5 KB a gene) and bit
+ * planes (row_len / 4 bytes for each of a gene's bins up to 16, at most 8 GiB). With a smaller workspace (at least
  * tenex_te_pairs_workspace_bytes) they use what fits, down to none: every pair then
  * runs in the shared-memory kernel. The tables start at the workspace's next multiple
  * of 256 bytes; an aligned workspace wastes none of it. */

@@ -997,12 +997,52 @@ int64_t col_bound(int n, int b_max) {
   return (int64_t)n * std::min(b * b, kMaxCols);
 }
 
+// A pair's cells (occupied target states x source bins) up to which the tensor cores are
+// the faster: their time goes with cells x samples, the counting kernel's with samples
+// plus, per cell, its own entropy pass. Measured, ms of both kernels with 900 / 1,050 /
+// 1,200 / 1,400 for the 1,200 below: 10,000 genes x 20,000 samples 637 / 637 / 634 / 638;
+// 2,000 x 5,000 7.10 / 7.14 / 7.22 / 7.34; 1,000 x 2,500 1.39 / 1.38 / 1.35 / 1.30; 301 x
+// 101,003 2.35 / 2.17 / 2.12 / 2.21. Short series: 2,000 x 600 (b to 16) at a limit of
+// 1,000 / 1,600 / 2,600 cells 4.82 / 4.19 / 3.76.
+int max_cells(double N) { return N <= 2078.0 ? 4096 : (int)(1200.0 * N / (N - 1470.0)); }
+
+// Whether a pair of b_max bins each is the tensor cores': then every pair is.
+bool takes_every_pair(int b_max, int N) {
+  const int64_t b = b_max;
+  return b * b <= kMaxCols && b * b * b <= max_cells(N);
+}
+
+// Whether a launch over `pairs` pairs is faster with the tensor-core path than in the
+// counting kernel alone. The path adds two launches and the plan's serial chain (25 us at
+// the least), the planes of all n genes however few the pairs, and an item's chain of
+// N / 256 steps; where only some pairs are its own the counting kernel runs after it, with
+// its own last round of items. The counting kernel takes pairs x (N + about 2,000) / 2.1e12
+// s where its items (32 sources of one target at the least) fill the SMs; up to 17 genes
+// the two chains are about equally long. Measured, us with the path / without, b_max 6 | b_max 16:
+//   genes x samples  100 x 300 46 / 36 | 86 / 64   200 x 300 68 / 67 | 129 / 125
+//   100 x 2,000 54 / 46 | 119 / 74   200 x 2,000 71 / 84 | 184 / 146
+//   300 x 2,000 87 / 150 | 271 / 261   140 x 20,000 102 / 189 | 323 / 263
+//   300 x 20,000 148 / 671 | 856 / 973   20 x 100,000 189 / 248 | 507 / 334
+//   10 x 1,000,000 1,320 / 1,140 | 3,570 / 2,020   20 x 1,000,000 1,530 / 2,200 | 5,230 / 3,460
+//   10,000 x 20,000, b_max 16, one target's pairs 1,010 / 204, 16 targets' 1,960 / 1,750,
+//   32 targets' 2,900 / 3,180; 2,000 x 20,000, b_max 6, 1 target 182 / 79, 8: 197 / 221.
+// Over 700 sizes (2 to 10,000 genes, 100 to 1,000,000 samples) the choice is on average
+// within 1% of the better one.
+bool worth_it(int n, int N, int b_max, int64_t pairs) {
+  const double work = (double)pairs * (N + 2000.0), planes = (double)n * N;
+  if (!takes_every_pair(b_max, N))
+    return work >= 1e8 + std::min(1.5e5 * N, 5e8) + 25.0 * planes;
+  const double items = ((double)pairs / (n - 1) + 1) * ((n + 31) / 32), sms = 148;
+  return pairs >= 300 && work * std::max(1.0, sms / items) >= 1e8 + 5.0 * planes;
+}
+
 }  // namespace
 
 // Plane rows for every gene up to 16 bins; sources of more bins use what those leave.
 // 8 GiB of planes at most (22,000 genes of 16 bins x 100,000 cells).
 int64_t te_mma_bytes(int n, int64_t row_len, int b_max) {
   if (row_len >= ((int64_t)1 << 24)) return 0;  // float32 counts are exact below 2^24
+  if (!worth_it(n, (int)row_len - 1, b_max, (int64_t)n * (n - 1))) return 0;
   const int64_t plane = round_up(row_len, 256) / 8 * 2;
   int64_t rows = (int64_t)n * std::min(b_max, kMaxTgtBins);
   rows = std::min(rows, ((int64_t)8 << 30) / plane);
@@ -1011,7 +1051,8 @@ int64_t te_mma_bytes(int n, int64_t row_len, int b_max) {
 
 bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
   M->cap_rows = 0;
-  if (M->row_len >= ((int64_t)1 << 24)) return false;
+  if (M->row_len >= ((int64_t)1 << 24) || !worth_it(M->n, M->N, M->b_max, M->p1 - M->p0))
+    return false;
   const int n = M->n;
   // work items are counted in 32 bits: at most one per target and pair of source tiles (a
   // full tile has over kRows - bins rows). Beyond 170,000 genes of 16 bins.
@@ -1044,15 +1085,7 @@ bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
   M->grp = reinterpret_cast<uint32_t*>(take((int64_t)n * 64));
   M->colq = reinterpret_cast<float2*>(take(cols * 16));
   M->colrow = reinterpret_cast<int2*>(M->colq + cols);
-  // A pair's cells (occupied target states x source bins) up to which the tensor cores
-  // are the faster: their time goes with cells x samples, the counting kernel's with
-  // samples plus, per cell, its own entropy pass. Measured, ms of both kernels with 900 /
-  // 1,050 / 1,200 / 1,400 for the 1,200 below: 10,000 genes x 20,000 samples 637 / 637 /
-  // 634 / 638; 2,000 x 5,000 7.10 / 7.14 / 7.22 / 7.34; 1,000 x 2,500 1.39 / 1.38 / 1.35 /
-  // 1.30; 301 x 101,003 2.35 / 2.17 / 2.12 / 2.21. Short series: 2,000 x 600 (b to 16) at
-  // a limit of 1,000 / 1,600 / 2,600 cells 4.82 / 4.19 / 3.76.
-  const double N = M->N;
-  M->max_cells = N <= 2078.0 ? 4096 : (int)(1200.0 * N / (N - 1470.0));
+  M->max_cells = max_cells(M->N);
   M->cap_rows = std::min<int64_t>(rows, (int64_t)1 << 29);
   M->P = reinterpret_cast<uint32_t*>(at);
   M->F = M->P + M->cap_rows * M->words;
@@ -1060,8 +1093,7 @@ bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
 }
 
 bool te_mma_takes_all(const TeMma& M) {
-  const int64_t b = M.b_max;
-  return b * b <= kMaxCols && b * b * b <= M.max_cells && (int64_t)M.n * b <= M.cap_rows;
+  return takes_every_pair(M.b_max, M.N) && (int64_t)M.n * M.b_max <= M.cap_rows;
 }
 
 int te_mma_launch(const TeMma& M, const DevAttr& A, bool pair_list, cudaStream_t stream) {

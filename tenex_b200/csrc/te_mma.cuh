@@ -60,11 +60,12 @@ struct TeMma {
 };
 
 // Bytes behind the workspace's base part that the tensor-core path would use for
-// every gene (0: it does not apply to such series or bin counts).
+// every gene (0: it does not apply to such series, or is not the faster even for all
+// pairs of them).
 int64_t te_mma_bytes(int n, int64_t row_len, int b_max);
 
 // Lays the path's buffers out in `bytes` bytes at `mem` (256-byte aligned): true
-// when there is room for it.
+// when there is room for it and the launch has enough pairs.
 bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes);
 
 // Enqueues validation, source order and, with M.cap_rows > 0, the plan, the bit

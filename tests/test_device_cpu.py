@@ -14,8 +14,8 @@ def test_to_device_takes_a_tensor_that_requires_grad():
 
 def test_workspace_falls_back_to_the_least_when_memory_is_short(monkeypatch):
     L = native.lib()
-    full = L.tenex_te_workspace_bytes(200, 3000, 16)
-    least = L.tenex_te_pairs_workspace_bytes(200, 3000, 16)
+    full = L.tenex_te_workspace_bytes(1000, 3000, 16)
+    least = L.tenex_te_pairs_workspace_bytes(1000, 3000, 16)
     assert full > least
     real, asked = torch.empty, []
 
@@ -26,8 +26,18 @@ def test_workspace_falls_back_to_the_least_when_memory_is_short(monkeypatch):
         return real(nb, **kw)
 
     monkeypatch.setattr(torch, "empty", empty)
-    assert D.workspace("cpu", 200, 3000, 16).numel() == least and asked == [full, least]
+    assert D.workspace("cpu", 1000, 3000, 16).numel() == least and asked == [full, least]
     monkeypatch.setattr(torch, "empty", lambda *a, **k: (_ for _ in ()).throw(
         torch.OutOfMemoryError("no room")))
     with pytest.raises(torch.OutOfMemoryError):
-        D.workspace("cpu", 200, 3000, 16)
+        D.workspace("cpu", 1000, 3000, 16)
+
+
+def test_workspace_of_small_problems_is_the_least():
+    """Few genes, whatever the series' length, run without the tensor-core path: their
+    workspace holds none of its tables and planes."""
+    L = native.lib()
+    for n, T, b in ((2, 2, 2), (2, 16_000_000, 16), (20, 1_000_000, 16), (60, 1000, 16)):
+        assert L.tenex_te_workspace_bytes(n, T, b) < L.tenex_te_pairs_workspace_bytes(n, T, b) + 256
+    for n, T, b in ((20, 1_000_000, 6), (300, 2000, 6), (2000, 5000, 16), (10_000, 20_000, 38)):
+        assert L.tenex_te_workspace_bytes(n, T, b) > L.tenex_te_pairs_workspace_bytes(n, T, b) + n * T // 8

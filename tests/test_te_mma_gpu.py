@@ -165,7 +165,7 @@ def test_targets_of_many_bins_and_few_states(cuda, wide):
     `wide`, beside targets of many states."""
     rng = np.random.default_rng(40 + wide)
     T, rows, npv = 400, [], []
-    for b in (8, 9, 11, 16):
+    for b in (8, 9, 11, 16) * 10:
         for v0, v1 in ((0, 0), (b - 1, b - 1), (0, 1), (b - 2, b - 1), (0, b - 1), (b // 2, 1)):
             rows.append(np.where(rng.random(T) < 0.4, v0, v1))
             npv.append(b)
@@ -184,7 +184,7 @@ def test_targets_of_many_bins_and_few_states(cuda, wide):
                                    (300, 292)])
 def test_lag_close_to_the_length(cuda, T, lag):
     """Dense genes of 8 to 16 bins with T - lag from 1 to 10: fewer samples than bins."""
-    bins, npv, bmax = _bins(1000 * T + lag, 70, T, 8, 16)
+    bins, npv, bmax = _bins(1000 * T + lag, 250, T, 8, 16)
     _all_outputs_match_oracle(bins[:, :, 0].astype(np.uint8), npv, bmax, lag, cuda)
 
 
@@ -192,8 +192,8 @@ def test_lag_close_to_the_length(cuda, T, lag):
 def test_engine_with_a_lag_close_to_the_length(cuda, T, tau):
     from tenex_b200 import TransferEntropyEngine
     rng = np.random.default_rng(T)
-    x = np.log1p(rng.poisson(3.0, (60, T)) * (rng.random((60, T)) < 0.7)).astype(np.float32)
-    res = TransferEntropyEngine(x, np.array([f"g{i}" for i in range(60)])).compute(
+    x = np.log1p(rng.poisson(3.0, (240, T)) * (rng.random((240, T)) < 0.7)).astype(np.float32)
+    res = TransferEntropyEngine(x, np.array([f"g{i}" for i in range(240)])).compute(
         accelerator="gpu", tau=tau, kp=0.5)
     ref = O.te_matrix(np.asarray(res.bin_arrs), np.asarray(res.n_per_var), tau=tau)
     assert np.max(np.abs(res.matrix - ref)) <= TOL
@@ -262,7 +262,7 @@ def test_error_is_no_larger_than_the_counting_kernels(cuda, bt, bs):
 
 
 @pytest.mark.parametrize("n,T,b", [(260, 300, (2, 16)), (300, 1200, (2, 12)),
-                                   (250, 2000, (2, 38)), (230, 70000, (2, 24))])
+                                   (340, 2000, (2, 38)), (230, 70000, (2, 24))])
 def test_value_of_a_pair_is_the_same_by_every_route(cuda, n, T, b):
     """Tensor cores or shared-memory counters of 32 or 16 bits, any launch shape, pair range
     or list: the terms of a column are added in one order in float32, all else in
@@ -285,3 +285,81 @@ def test_value_of_a_pair_is_the_same_by_every_route(cuda, n, T, b):
     tgt, loc = ids // (n - 1), ids % (n - 1)
     pl = te_pair_list(db, npv_t, bmax, 1, np.stack((tgt, loc + (loc >= tgt)), 1))
     assert torch.equal(te[torch.as_tensor(ids, device=cuda)], pl)
+
+
+def _items(ws):
+    """Work items of the tensor-core launch that used this workspace (0: there was none)."""
+    return int(ws[16:20].view(torch.int32))
+
+
+# the edges of SHAPES, with the genes that make the tensor-core path worth its launches
+@pytest.mark.parametrize("n,T,b,lag", [
+    (230, 2, (1, 3), 1), (230, 65, (2, 4), 1), (230, 256, (2, 2), 1), (230, 257, (2, 5), 1),
+    (231, 320, (3, 7), 33), (240, 769, (2, 9), 1), (231, 1024, (4, 4), 1),
+    (330, 1030, (2, 16), 3), (340, 1500, (13, 16), 1), (360, 2049, (2, 38), 300),
+    (300, 700, (5, 38), 1)])
+@pytest.mark.parametrize("skew", [False, True])
+def test_counts_and_te_of_enough_genes(cuda, n, T, b, lag, skew):
+    bins, npv, bmax = _bins(n * T + skew, n, T, *b, skew=skew)
+    bmax = max(bmax, b[1])            # declared, so that the size decides and not the draw
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P, s = n * (n - 1), native.stream_ptr()
+    ref = O.te_pairfree(bins, npv, tau=lag)
+    ws = D.workspace(cuda, n, db.row_len, bmax)
+    m = torch.zeros((n, n), dtype=torch.float32, device=cuda)
+    native.call("tenex_te_pairfree", db.ptr(), db.ld, npv_t.data_ptr(), bmax, n, db.row_len, lag,
+                0, P, m.data_ptr(), native.OUT_MATRIX, n, ws.data_ptr(), ws.numel(), None, s)
+    native.call("tenex_workspace_status", ws.data_ptr(), s)
+    assert _items(ws) > 0 and not bool(m.diagonal().any())
+    te = _run(db, npv_t, bmax, lag, 0, P, cuda, True).cpu().numpy()
+    assert np.max(np.abs(te - ref)) <= TOL
+    assert np.array_equal(m.cpu().numpy().T[~np.eye(n, dtype=bool)], te)
+    for p0, cnt in ((P // 9, P - P // 5), (P // 2, n // 2)):  # ranges that cut targets
+        part = _run(db, npv_t, bmax, lag, p0, cnt, cuda, True).cpu().numpy()
+        assert np.array_equal(part, te[p0:p0 + cnt])
+    if P * bmax ** 3 <= 60_000_000:
+        c = [torch.full((P, bmax ** 3), -1, dtype=torch.int32, device=cuda) for _ in range(2)]
+        t = [_run(db, npv_t, bmax, lag, 0, P, cuda, tc, counts=k).cpu().numpy()
+             for tc, k in zip((True, False), c)]
+        assert torch.equal(c[0], c[1])
+        assert np.array_equal(t[0], te) and np.array_equal(t[1], te)
+
+
+def test_counts_of_tensor_cores_exact_up_to_2_pow_24(cuda):
+    """float32 accumulators hold every count of the longest series the path takes; twenty
+    genes of it are enough work."""
+    T, n = (1 << 24) - 3, 20
+    rng = np.random.default_rng(8)
+    x = np.zeros((n, T), np.uint8)
+    for i in range(1, n):
+        x[i] = rng.random(T) < (0.5, 1e-6, 1 - 1e-6)[i % 3]
+        x[i, i], x[i, i + 20] = 0, 1
+    npv = np.array([1] + [2] * (n - 1), np.int32)
+    db = D.pack_bins(x, cuda)
+    npv_t = torch.as_tensor(npv, device=cuda)
+    P = n * (n - 1)
+    c = [torch.zeros((P, 8), dtype=torch.int32, device=cuda) for _ in range(2)]
+    te = [_run(db, npv_t, 2, 1, 0, P, cuda, tc, counts=k) for tc, k in zip((True, False), c)]
+    assert D.workspace(cuda, n, db.row_len, 2).numel() > n * T // 2   # with room for planes
+    assert torch.equal(c[0], c[1]) and int(c[0].sum(1).min()) == T - 1
+    assert float((te[0] - te[1]).abs().max()) <= TOL
+
+
+def test_small_launches_run_without_the_tensor_cores(cuda):
+    """Few genes and ranges of few pairs go to the counting kernel alone (its ticket says
+    so: no work item of the other path), which is the faster there, with equal results."""
+    for n, T, b, cnt in ((40, 2000, (2, 6), None), (10, 60_000, (2, 16), None),
+                         (800, 3000, (2, 16), 300)):
+        bins, npv, bmax = _bins(n, n, T, *b)
+        db = D.pack_bins(bins, cuda)
+        npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+        P = n * (n - 1) if cnt is None else cnt
+        ws = torch.empty(64 << 20, dtype=torch.uint8, device=cuda)
+        out = torch.zeros(P, dtype=torch.float32, device=cuda)
+        native.call("tenex_te_pairfree", db.ptr(), db.ld, npv_t.data_ptr(), bmax, n, db.row_len,
+                    1, 0, P, out.data_ptr(), native.OUT_PAIRFREE, 0, ws.data_ptr(), ws.numel(),
+                    None, native.stream_ptr())
+        assert _items(ws) == 0
+        ref = O.te_pairfree(bins, npv, 1, 0, P)
+        assert np.max(np.abs(out.cpu().numpy() - ref)) <= TOL
