@@ -58,14 +58,17 @@ typedef struct {
 } tenex_dev_info;
 
 /* Launch shape of the persistent histogram kernels (0 fields, or a NULL config,
- * = defaults: 2 CTAs x 512 threads per SM, 512 sources per item; when the
- * largest pair's histogram does not fit two CTAs per SM, one CTA per SM, of
- * 1024 threads if neither threads nor ctas_per_sm was given). */
+ * = defaults: 2 CTAs x 512 threads per SM; when the largest pair's histogram
+ * does not fit two CTAs per SM, one CTA per SM, of 1024 threads if neither
+ * threads nor ctas_per_sm was given). A pair's TE does not depend on the shape,
+ * except where it decides whether the pair's histogram fits shared memory. */
 typedef struct {
   int threads;      /* threads per CTA: 128, 256, 512 or 1024          */
   int ctas_per_sm;  /* resident CTAs per SM (grid = sm_count * this)    */
-  int src_chunk;    /* sources per work item (one target per item);
-                       0: n_vars / 12, at least 32 and at most 512     */
+  int src_chunk;    /* sources per work item (one target per item); 0: a
+                       twelfth of n_vars, fewer where the pair range has few
+                       targets, but no more than n_vars / 32 items a target,
+                       and at most 512; pair lists: as item_start has them */
   int smem_bytes;   /* dynamic shared memory per CTA (0 = fill the SM)  */
 } tenex_te_config;
 

@@ -207,9 +207,16 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // Arrival on the same barrier of the cluster's CTA `cta` (which may be this one), for
-// what this CTA wrote for the tensor cores (ordered before by its proxy fences). A
-// release at cluster scope would wait for every load of this thread in flight, about
-// 1,000 cycles.
+// what this CTA wrote to its own shared memory for the tensor cores. Why those writes
+// are in place when the other CTA's MMA has this SM read them: each writing thread has
+// passed fence.proxy.async.shared::cta, which makes its writes visible to the async
+// proxy of this shared memory, and the warp has synchronised, before one lane arrives;
+// the MMA is issued only after the barrier's phase shows that arrival, and it reads this
+// CTA's part through this SM's own async proxy. No other copy of shared memory exists
+// that could be older. The arrival's default release is of CTA scope, so this rests on the
+// fence and on shared memory being one memory, not on cluster-scope synchronisation; a
+// release at cluster scope would also wait for every global load of this thread in
+// flight, about 1,000 cycles a step.
 __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta) {
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(bar)), "r"(cta));

@@ -995,8 +995,8 @@ static int plan_te_launch(const TeParams& P, const tenex_te_config* cfg, const D
   // Default shape: 2 CTAs x 512 threads per SM. When the largest histogram needs
   // the shared memory of a whole SM (b_max ~ 32 and above) the loop below drops
   // to one CTA per SM; with both left to the library the CTA then takes 1024
-  // threads, so an SM keeps 32 warps (10,000 genes x 20,000 cells, b_max 38:
-  // 989 ms against 1055 ms for one 512-thread CTA).
+  // threads, so an SM keeps 32 warps (10,000 genes x 20,000 cells, b_max 38, when
+  // every pair was counted here: 989 ms against 1055 ms for one 512-thread CTA).
   const bool auto_shape = !(cfg && (cfg->threads || cfg->ctas_per_sm));
   int threads = (cfg && cfg->threads) ? cfg->threads : 512;
   int cps = (cfg && cfg->ctas_per_sm) ? cfg->ctas_per_sm : 2;  // lowered below if slots do not fit
@@ -1216,15 +1216,16 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   P.lag = (int)lag;
   P.p0 = p0;
   P.p1 = p0 + n_pairs;
-  // Sources per item: a twelfth of them (32 at least, 512 at most). Sources are ordered
-  // by bin count and an item's slots are sized for its widest source, so a chunk should
-  // span few bin counts; below 100 sources the target's staging shows, above 512 the rows
-  // of a chunk no longer share L2. Measured at 512 / 250 / this rule, ms: 1,000 x 5,000
-  // (b to 32) 8.89 / 7.88 / 7.3, 2,000 x 5,000 (b to 16) 7.35 / 7.19 / 7.15, 2,500 x
-  // 10,000 (b to 32) 55.0 / 53.7 / 53.7; 10,000 x 20,000 at 256 / 512 / 768: 643 / 635 /
-  // 638. Fewer still where there are too few targets for 16 items per CTA (few genes, a
-  // short pair range): the items are uneven, and one round of them leaves most SMs idle
-  // at its end (301 genes x 101,003 samples: 1.88 -> 0.64 ms for the pairs counted here).
+  // Sources per item: a twelfth of them, 512 at most. Sources are ordered by bin count and
+  // an item's slots are sized for its widest source, so a chunk should span few bin counts;
+  // above 512 the rows of a chunk no longer share L2. Measured at 512 / 250 / this rule,
+  // ms: 1,000 x 5,000 (b to 32) 8.89 / 7.88 / 7.3, 2,000 x 5,000 (b to 16) 7.35 / 7.19 /
+  // 7.15, 2,500 x 10,000 (b to 32) 55.0 / 53.7 / 53.7; 10,000 x 20,000 at 256 / 512 / 768:
+  // 643 / 635 / 638. Fewer where there are too few targets for 16 items per CTA (few genes,
+  // a short pair range), down to 32 or, since the chunks are equal, a little less: the
+  // items are uneven, and one round of them leaves most SMs idle at its end (301 genes x
+  // 101,003 samples: 1.88 -> 0.64 ms for the pairs counted here). Below that the target's
+  // staging shows.
   P.W = (cfg && cfg->src_chunk) ? cfg->src_chunk : 512;
   if (!pairs && !(cfg && cfg->src_chunk)) {
     const int64_t targets = (p0 + n_pairs - 1) / (n - 1) - p0 / (n - 1) + 1;

@@ -8,7 +8,7 @@ keep working. Behind it every kernel calls libtenex_sm100.so (sm_100a); there
 is no CPU or library fallback.
 
 Priority (highest first):
-  1. GEMM-B2       — binary data (b_max = 2), no source filter: tcgen05 INT8 GEMM
+  1. GEMM-B2       — binary data (b_max = 2), no source filter: tcgen05 GEMM
   2. Full-SMEM     — b_max^3 <= 65536 and the reference's SMEM formula fits
   3. Adaptive-SMEM — any b_max (bins coarsened to the device's shared-memory limit)
 """

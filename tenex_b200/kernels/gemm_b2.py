@@ -58,7 +58,8 @@ def tile_width(n: int) -> int:
 
 
 class GEMMB2Kernel(TEKernel):
-    """Exact binary TE for all pairs from three INT8 tensor-core contractions."""
+    """Exact binary TE for all pairs from three tensor-core contractions (4-bit or
+    INT8 operands)."""
 
     @property
     def name(self) -> str:
@@ -101,4 +102,4 @@ class GEMMB2Kernel(TEKernel):
         return self.compute_matrix(data, n_vars, tau, torch.device("cuda", ids[0]), **kwargs)
 
     def log_description(self, **kwargs) -> str:
-        return "GEMM-B2 (tcgen05 INT8 contractions + fused TE epilogue, exact)"
+        return "GEMM-B2 (tcgen05 contractions + fused TE epilogue, exact)"
