@@ -60,10 +60,15 @@ _copy_workers = max(1, min(8, os.cpu_count() or 1))
 _copy_pool_lock = threading.Lock()
 _STAGE_BYTES = 32 << 20        # one staging chunk of the host -> device copy
 # Smaller arrays take the plain pageable copy (ms, plain / staged: to the device 16 MB
-# 0.87 / 1.70, 40 MB 2.1 / 2.7, 100 MB 8.6 / 4.7; back 6 MB 0.35 / 1.16, 16 MB 0.85 /
-# 1.43, 40 MB 21.5 / 3.7, where the destination's fresh pages are touched one by one)
+# 0.87 / 1.70, 40 MB 2.1 / 2.7, 100 MB 8.6 / 4.7). Back, a plain copy is the faster into
+# memory that the process used before and the slower into fresh pages, which the driver
+# touches one by one; into a numpy array, of huge pages where the system has them, and with
+# its pages touched first, in between (ms, used / fresh memory, staged 6 MB 1.2 / 1.0, 16 MB
+# 1.4 / 1.9; plain into a torch tensor 0.35 / 2.7, 0.85 / 7.7; into a touched array 0.4 /
+# 0.8, 1.1 / 3.2; 40 MB staged 3.0 / 4.3, touched 2.7 / 15)
 _DIRECT_BYTES = 48 << 20
 _DIRECT_HOST_BYTES = 20 << 20
+_TOUCH_BYTES = 1 << 20         # below this the touching costs what it saves
 
 
 def _pool():
@@ -144,8 +149,13 @@ def to_host(t: torch.Tensor) -> np.ndarray:
         return t.numpy()
     t = t.contiguous()
     nbytes = t.numel() * t.element_size()
-    if nbytes < _DIRECT_HOST_BYTES:
+    if nbytes < _TOUCH_BYTES:
         return t.cpu().numpy()
+    if nbytes < _DIRECT_HOST_BYTES:
+        out = np.empty(tuple(t.shape), dtype=torch.empty(0, dtype=t.dtype).numpy().dtype)
+        out.reshape(-1).view(np.uint8)[::4096] = 0
+        torch.from_numpy(out).copy_(t)
+        return out
     flat = t.view(-1)
     numel = flat.numel()
     out = np.empty(numel, dtype=torch.empty(0, dtype=t.dtype).numpy().dtype)

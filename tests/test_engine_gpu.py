@@ -398,3 +398,16 @@ def test_binarize_takes_a_tensor_that_requires_grad(cuda):
     want = binarize(x, "mean", cuda)
     got = binarize(x.requires_grad_(), "mean", cuda)
     assert torch.equal(got[0].data, want[0].data) and torch.equal(got[3], want[3])
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.int8, torch.int32, torch.float32,
+                                   torch.float64])
+def test_to_host_at_the_sizes_where_its_way_changes(cuda, dtype):
+    size = torch.empty(0, dtype=dtype).element_size()
+    for nbytes in (0, 8, 4096, (1 << 20) - 8, 1 << 20, (1 << 20) + 8, (20 << 20) - 8, 20 << 20,
+                   (33 << 20) + 8):
+        t = torch.randint(0, 100, (2, nbytes // size // 2), device=cuda).to(dtype)
+        got = D.to_host(t)
+        assert got.shape == tuple(t.shape) and torch.equal(torch.from_numpy(got), t.cpu())
+    wide = torch.arange(3_000_000, device=cuda).to(dtype).view(1000, 3000)
+    assert np.array_equal(D.to_host(wide[:, :2001]), wide[:, :2001].cpu().numpy())
