@@ -81,6 +81,16 @@ def _pool():
         return _copy_pool
 
 
+def _forget_pool():
+    """In a forked child: the parent's copy threads do not exist here, and its lock may
+    have been held."""
+    global _copy_pool, _copy_pool_lock
+    _copy_pool, _copy_pool_lock = None, threading.Lock()
+
+
+os.register_at_fork(after_in_child=_forget_pool)
+
+
 def all_finite(a: np.ndarray) -> bool:
     """np.isfinite(a).all() for a large C-contiguous array, checked in one slab (of at
     most 4M elements) per host copy thread (ufuncs run without the GIL)."""

@@ -1,4 +1,8 @@
 """Host-side parts of the device layer that need no GPU."""
+import os
+import threading
+
+import numpy as np
 import pytest
 import torch
 
@@ -41,3 +45,22 @@ def test_workspace_of_small_problems_is_the_least():
         assert L.tenex_te_workspace_bytes(n, T, b) < L.tenex_te_pairs_workspace_bytes(n, T, b) + 256
     for n, T, b in ((20, 1_000_000, 6), (300, 2000, 6), (2000, 5000, 16), (10_000, 20_000, 38)):
         assert L.tenex_te_workspace_bytes(n, T, b) > L.tenex_te_pairs_workspace_bytes(n, T, b) + n * T // 8
+
+
+def test_finite_check_in_a_forked_process(monkeypatch):
+    """Arrays of a million elements are checked on host threads, which a forked child of a
+    process that has them does not have."""
+    monkeypatch.setattr(D, "_copy_workers", 8)
+    monkeypatch.setattr(D, "_copy_pool", None)
+    a = np.zeros(3 << 19)
+    assert D.all_finite(a)
+    ready = threading.Barrier(9)
+    tasks = [D._pool().submit(ready.wait, 20) for _ in range(8)]
+    ready.wait(20)
+    assert len([t.result() for t in tasks]) == 8          # all threads are up
+    assert D.all_finite(a)
+    pid = os.fork()
+    if pid == 0:
+        threading.Timer(20, os._exit, (3,)).start()
+        os._exit(0 if D.all_finite(a) and not D.all_finite(np.append(a, np.nan)) else 2)
+    assert os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]) == 0
