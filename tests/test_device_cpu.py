@@ -64,3 +64,21 @@ def test_finite_check_in_a_forked_process(monkeypatch):
         threading.Timer(20, os._exit, (3,)).start()
         os._exit(0 if D.all_finite(a) and not D.all_finite(np.append(a, np.nan)) else 2)
     assert os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]) == 0
+
+
+def test_permutations_are_sorted_one_by_one_when_memory_is_short(monkeypatch):
+    from tenex_b200.inference.surrogate_test import build_block_perm
+    want = build_block_perm(6, 400, "block", 10, 2, 9, 5, "cpu")[0]
+    real = torch.argsort
+
+    def argsort(x, **kw):
+        if x.shape[0] > 6:
+            raise torch.OutOfMemoryError("no room")
+        return real(x, **kw)
+
+    monkeypatch.setattr(torch, "argsort", argsort)
+    assert torch.equal(build_block_perm(6, 400, "block", 10, 2, 9, 5, "cpu")[0], want)
+    monkeypatch.setattr(torch, "argsort", lambda *a, **k: (_ for _ in ()).throw(
+        torch.OutOfMemoryError("no room")))
+    with pytest.raises(torch.OutOfMemoryError):
+        build_block_perm(6, 400, "block", 10, 2, 9, 5, "cpu")
