@@ -100,7 +100,9 @@ class SurrogateAccumulator:
         self.sum = torch.zeros((n, n), dtype=torch.float64, device=dev)
         self.sumsq = torch.zeros((n, n), dtype=torch.float64, device=dev)
         self.cnt = torch.zeros((n, n), dtype=torch.int32, device=dev)
-        self.ws = D.workspace(dev, n, db.row_len, self.b_max)
+        # the workspace takes room that the permutations may need: asked for by the first
+        # surrogate, when they are made
+        self.ws = None
         if binary:
             self.tmp = torch.zeros((n, n), dtype=torch.float32, device=dev)
             nb = int(native.lib().tenex_b2_workspace_bytes(n, db.row_len, tau * db.K))
@@ -117,6 +119,9 @@ class SurrogateAccumulator:
             native.call("tenex_stats_accumulate", self.tmp.data_ptr(), self.obs.data_ptr(),
                         self.sum.data_ptr(), self.sumsq.data_ptr(), self.cnt.data_ptr(), n, s)
         else:
+            if self.ws is None:
+                self.ws = D.workspace(self.shuf.data.device, self.db.n, self.db.row_len,
+                                      self.b_max)
             D.surrogate_accumulate(self.shuf, self.npv, self.b_max, self.tau, self.obs, self.sum,
                                    self.sumsq, self.cnt, self.p0, self.np_, cfg=self.cfg,
                                    ws=self.ws)
@@ -126,7 +131,7 @@ class SurrogateAccumulator:
         if self.binary:
             native.call("tenex_b2_status", self.b2ws.data_ptr(), self.db.n, self.shuf.row_len,
                         self.tau * self.db.K, s)
-        else:
+        elif self.ws is not None:
             native.call("tenex_workspace_status", self.ws.data_ptr(), s)
 
 

@@ -253,3 +253,22 @@ def test_block_shuffles_of_several_lengths_from_threads(cuda):
 
     with ThreadPoolExecutor(max_workers=4) as ex:
         assert all(ex.map(work, (1000, 90_000, 1500, 60_000)))
+
+
+@pytest.mark.parametrize("kernel,hi,asked", [("Full-SMEM", 7, ["permutations", "workspace"]),
+                                             ("GEMM-B2", 2, ["permutations"])])
+def test_permutations_come_before_the_workspace(cuda, monkeypatch, kernel, hi, asked):
+    """The workspace takes up to 8 GiB where there is room and little where there is not; what
+    the permutations need is allocated before. Binary data has no use for one."""
+    from tenex_b200.inference import surrogate_test as ST
+    order = []
+    perm, ws = ST.build_block_perm, D.workspace
+    monkeypatch.setattr(ST, "build_block_perm",
+                        lambda *a, **k: (order.append("permutations"), perm(*a, **k))[1])
+    monkeypatch.setattr(D, "workspace",
+                        lambda *a, **k: (order.append("workspace"), ws(*a, **k))[1])
+    bins, npv, bmax = O.remap(np.random.default_rng(3).integers(0, hi, (20, 300)).astype(np.int32))
+    obs = O.te_matrix(bins, npv).astype(np.float32)
+    s1, _, _ = ST.SurrogateTestMethod.accumulate(obs, cuda, bins.reshape(20, 300, 1), npv, bmax,
+                                                 kernel, 1, 3, "block", 20, 5)
+    assert order == asked and s1.any()
