@@ -32,19 +32,18 @@ def item_table(tgt_sorted: np.ndarray, run: int = 128) -> np.ndarray:
     return np.concatenate([items, [P]]).astype(np.int64)
 
 
-def te_source_rows(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: int,
-                   sources: np.ndarray, cfg=None, run: int = 128,
-                   check_data: bool = True) -> torch.Tensor:
-    """(n, n) float32 device matrix with [src, tgt] = TE(src -> tgt) for the distinct
-    gene indices `sources` and every target, 0 elsewhere and on the diagonal. The
+def te_source_block(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: int,
+                    sources: np.ndarray, cfg=None, run: int = 128,
+                    check_data: bool = True) -> torch.Tensor:
+    """(m, n) float32 device tensor with [k, tgt] = TE(sources[k] -> tgt) for the m distinct
+    gene indices `sources` and every target, 0 where the target is the source. The
     pair list (target-major, the sources in the given order, a source against itself
     included and dropped from the result) is a regular grid, so it and its items are
     made on the device: 150 sources x 2,003 targets host to host 23 -> 3.5 ms."""
     dev = db.data.device
     n, m = db.n, len(sources)
-    out = torch.zeros((n, n), dtype=torch.float32, device=dev)
     if m == 0:
-        return out
+        return torch.zeros((0, n), dtype=torch.float32, device=dev)
     src = torch.as_tensor(np.ascontiguousarray(sources, dtype=np.int64)).to(dev)
     pairs = torch.empty((n, m, 2), dtype=torch.int64, device=dev)
     pairs[:, :, 0] = torch.arange(n, device=dev)[:, None]
@@ -61,8 +60,34 @@ def te_source_rows(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: int,
                 te.data_ptr(), ws.data_ptr(), ws.numel(), D._cfg(cfg), s)
     if check_data:
         native.call("tenex_workspace_status", ws.data_ptr(), s)
-    out[src] = te.t()
-    out[src, src] = 0.0
+    te[src, torch.arange(m, device=dev)] = 0.0
+    return te.t()
+
+
+def te_source_rows(db: D.DeviceBins, npv: torch.Tensor, b_max: int, tau: int,
+                   sources: np.ndarray, cfg=None, run: int = 128,
+                   check_data: bool = True) -> torch.Tensor:
+    """(n, n) float32 device matrix: te_source_block's rows at their sources, 0 elsewhere."""
+    block = te_source_block(db, npv, b_max, tau, sources, cfg, run, check_data)
+    return _rows_to_matrix(block, sources)
+
+
+def source_block_to_host(block: torch.Tensor, sources: np.ndarray) -> np.ndarray:
+    """The same matrix of a te_source_block on the host. Put together there where the device
+    holds the rows but not the (n, n) matrix (200,000 genes: 160 GB)."""
+    try:
+        m = _rows_to_matrix(block, sources)
+    except torch.OutOfMemoryError:
+        out = np.zeros((block.shape[1], block.shape[1]), dtype=np.float32)
+        out[sources] = D.to_host(block)
+        return out
+    return D.to_host(m)
+
+
+def _rows_to_matrix(block: torch.Tensor, sources: np.ndarray) -> torch.Tensor:
+    n = block.shape[1]
+    out = torch.zeros((n, n), dtype=torch.float32, device=block.device)
+    out[torch.as_tensor(np.ascontiguousarray(sources, dtype=np.int64)).to(block.device)] = block
     return out
 
 

@@ -293,11 +293,12 @@ class TransferEntropyEngine:
                 rm[pairs[:, 0], pairs[:, 1]] = te_h
                 self._result_matrix = rm.T.copy()
             else:
-                from tenex_b200.kernels.pair_list import te_source_rows
-                m = te_source_rows(work, npv_w, b_max_w, tau, self._source_indices(),
-                                   cfg=getattr(kobj, "cfg", None))
+                from tenex_b200.kernels.pair_list import source_block_to_host, te_source_block
+                src = self._source_indices()
+                block = te_source_block(work, npv_w, b_max_w, tau, src,
+                                        cfg=getattr(kobj, "cfg", None))
                 mark(6)
-                self._result_matrix = D.to_host(m)
+                self._result_matrix = source_block_to_host(block, src)
         else:
             info.update(mode="pairfree", pair_free=True)
             if len(device_ids) > 1:

@@ -411,3 +411,24 @@ def test_to_host_at_the_sizes_where_its_way_changes(cuda, dtype):
         assert got.shape == tuple(t.shape) and torch.equal(torch.from_numpy(got), t.cpu())
     wide = torch.arange(3_000_000, device=cuda).to(dtype).view(1000, 3000)
     assert np.array_equal(D.to_host(wide[:, :2001]), wide[:, :2001].cpu().numpy())
+
+
+def test_source_filter_without_room_for_the_matrix_on_the_device(cuda, monkeypatch):
+    """compute() with a source filter needs the sources' rows on the device; the (n, n) matrix
+    may be larger than what it has left."""
+    rng = np.random.default_rng(8)
+    x = np.log1p(rng.poisson(2.0, (40, 300))).astype(np.float32)
+    names = np.array([f"g{i:02d}" for i in range(40)])
+    eng = TransferEntropyEngine(x, names, sources=names[[3, 17, 30]])
+    want = eng.compute(accelerator="gpu").matrix
+    real, refused = torch.zeros, []
+
+    def zeros(*size, **kw):
+        if size == ((40, 40),) and torch.device(kw.get("device", "cpu")).type == "cuda":
+            refused.append(size)
+            raise torch.OutOfMemoryError("no room")
+        return real(*size, **kw)
+
+    monkeypatch.setattr(torch, "zeros", zeros)
+    got = eng.compute(accelerator="gpu").matrix
+    assert refused and np.array_equal(got, want) and want[[3, 17, 30]].any()
