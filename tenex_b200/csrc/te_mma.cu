@@ -1013,7 +1013,7 @@ bool takes_every_pair(int b_max, int N) {
 }
 
 // Whether a launch over `pairs` pairs is faster with the tensor-core path than in the
-// counting kernel alone. The path adds two launches and the plan's serial chain (25 us at
+// counting kernel alone, with room for its planes. The path adds two launches and the plan's serial chain (25 us at
 // the least), the planes of all n genes however few the pairs, and an item's chain of
 // N / 256 steps; where only some pairs are its own the counting kernel runs after it, with
 // its own last round of items. The counting kernel takes pairs x (N + about 2,000) / 2.1e12
@@ -1034,6 +1034,20 @@ bool worth_it(int n, int N, int b_max, int64_t pairs) {
     return work >= 1e8 + std::min(1.5e5 * N, 5e8) + 25.0 * planes;
   const double items = ((double)pairs / (n - 1) + 1) * ((n + 31) / 32), sms = 148;
   return pairs >= 300 && work * std::max(1.0, sms / items) >= 1e8 + 5.0 * planes;
+}
+
+// The same where the workspace has room for a part of the plane rows only: `room` is that
+// part of the most rows the genes can have. Genes have about half of the most bins, and the
+// counting kernel still runs after the path, so about min(1, 2 room)^2 of the pairs have to
+// be worth what the path adds. Measured, us without / with room for 0.07, 0.15, 0.25, 0.4,
+// 0.75 of the rows:
+//   100 x 20,000 (b to 6)   130 / 188, 196, 193, 164, 105   200 x 2,000 (6)  90 / 122, 119, 115, 105, 87
+//   300 x 5,000 (6)         238 / 276, 265, 244, 213, 106   400 x 3,000 (16) 497 / 518, 499, 473, 433, 408
+//   600 x 2,000 (6)         480 / 506, 475, 438, 357, 161   1,000 x 5,000 (16) 3,209 / 3,130, 2,898, 2,643, ...
+// Up to a twentieth short (tables moved to an aligned address) counts as all.
+bool worth_it_with(double room, int N, int64_t pairs) {
+  const double share = std::min(1.0, 2.0 * room);
+  return room >= 0.95 || (double)pairs * (N + 2000.0) * share * share >= 2.5e8;
 }
 
 }  // namespace
@@ -1064,6 +1078,8 @@ bool te_mma_layout(TeMma* M, unsigned char* mem, int64_t bytes) {
   const int64_t fixed = tables_bytes(n) + round_up(cols * 16, 256) + 256;
   const int64_t rows = (bytes - fixed) / ((int64_t)M->words * 8);
   if (bytes < fixed || rows < 2) return false;
+  const double most = (double)n * std::min(M->b_max, kMaxTgtBins);
+  if (!worth_it_with((double)rows / most, M->N, M->p1 - M->p0)) return false;
   unsigned char* at = mem;
   auto take = [&](int64_t b) {
     unsigned char* p = at;

@@ -363,3 +363,26 @@ def test_small_launches_run_without_the_tensor_cores(cuda):
         assert _items(ws) == 0
         ref = O.te_pairfree(bins, npv, 1, 0, P)
         assert np.max(np.abs(out.cpu().numpy() - ref)) <= TOL
+
+
+@pytest.mark.parametrize("b_hi", [7, 16, 38])
+@pytest.mark.parametrize("part,taken", [(0.02, False), (0.3, True), (0.55, True), (0.9, True)])
+def test_part_of_the_workspace_is_used_where_it_is_worth_it(cuda, b_hi, part, taken):
+    """Room for a few genes' bit planes only: the path's launches take longer than they
+    save, so the counting kernel runs alone; with room for more the planes are cut inside a
+    class of one bin count."""
+    n, T = 500, 1200
+    bins, npv, bmax = _bins(b_hi + 1, n, T, 2, b_hi)
+    bmax = max(bmax, b_hi)
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P, s = n * (n - 1), native.stream_ptr()
+    out = torch.zeros(P, dtype=torch.float32, device=cuda)
+    planes = n * min(bmax, 16) * (1280 // 8 * 2)            # the part that holds bit planes
+    nb = D.workspace(cuda, n, db.row_len, bmax).numel() - int(planes * (1 - part)) // 4 * 4
+    ws = torch.empty(nb, dtype=torch.uint8, device=cuda)
+    native.call("tenex_te_pairfree", db.ptr(), db.ld, npv_t.data_ptr(), bmax, n, db.row_len, 1,
+                0, P, out.data_ptr(), native.OUT_PAIRFREE, 0, ws.data_ptr(), nb, None, s)
+    native.call("tenex_workspace_status", ws.data_ptr(), s)
+    assert (_items(ws) > 0) == taken
+    assert np.max(np.abs(out.cpu().numpy() - O.te_pairfree(bins, npv, tau=1))) <= TOL
