@@ -386,3 +386,59 @@ def test_part_of_the_workspace_is_used_where_it_is_worth_it(cuda, b_hi, part, ta
     native.call("tenex_workspace_status", ws.data_ptr(), s)
     assert (_items(ws) > 0) == taken
     assert np.max(np.abs(out.cpu().numpy() - O.te_pairfree(bins, npv, tau=1))) <= TOL
+
+
+def test_captured_launch_and_two_streams(cuda):
+    """The tensor-core path in a CUDA graph replayed on other bins, and from two threads with
+    a stream and a workspace each: the values of an eager call."""
+    import threading
+    n, T, lag = 320, 1100, 1
+    sets = [_bins(seed, n, T, 2, 12) for seed in (1, 2)]
+    bmax = 12
+    dbs = [D.pack_bins(b, cuda) for b, _, _ in sets]
+    npvs = [torch.as_tensor(p, dtype=torch.int32, device=cuda) for _, p, _ in sets]
+    P = n * (n - 1)
+    want = [_run(d, p, bmax, lag, 0, P, cuda, True) for d, p in zip(dbs, npvs)]
+    assert not torch.equal(want[0], want[1])
+
+    def call(db, npv, out, ws):
+        native.call("tenex_te_pairfree", db.ptr(), db.ld, npv.data_ptr(), bmax, n, db.row_len,
+                    lag, 0, P, out.data_ptr(), native.OUT_PAIRFREE, 0, ws.data_ptr(), ws.numel(),
+                    None, native.stream_ptr())
+
+    ws = D.workspace(cuda, n, dbs[0].row_len, bmax)
+    db, npv, out = D.pack_bins(sets[0][0], cuda), npvs[0].clone(), torch.zeros_like(want[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(db, npv, out, ws)
+    for k in (0, 1, 0):
+        db.data.copy_(dbs[k].data)
+        npv.copy_(npvs[k])
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert _items(ws) > 0 and torch.equal(out, want[k])
+
+    got = [torch.zeros_like(w) for w in want]
+    failed = []
+
+    def work(k):
+        try:
+            torch.cuda.set_device(cuda)
+            s = torch.cuda.Stream(cuda)
+            with torch.cuda.stream(s):
+                mine = D.workspace(cuda, n, dbs[k].row_len, bmax)
+                for _ in range(20):
+                    call(dbs[k], npvs[k], got[k], mine)
+                native.call("tenex_workspace_status", mine.data_ptr(), native.stream_ptr())
+            s.synchronize()
+        except Exception as e:  # shown by the assertion below
+            failed.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(k,)) for k in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed and all(torch.equal(g, w) for g, w in zip(got, want))
