@@ -129,7 +129,7 @@ def measured_peaks() -> dict:
 
 
 def profile_traffic():
-    """DRAM bytes per launch of the TE kernel from the committed ncu summary."""
+    """DRAM bytes per all-pairs launch (both histogram kernels) from the committed ncu summary."""
     p = os.path.join(ROOT, "profiles", "te_pair_tile_cfg4.json")
     if os.path.exists(p):
         with open(p) as f:
@@ -328,28 +328,32 @@ def run_ours(args) -> None:
             dist.destroy_process_group()
         return
 
-    # ---- roofline of the dominant kernel (te_pair_tile_kernel) ----
+    # ---- the launch against what counting every pair would take ----
     N = C - TAU
-    incr = (p1 - p0) * N                                   # histogram increments per launch
+    incr = (p1 - p0) * N                                   # samples of pairs per launch
     peak_atomic = max(native.probe_smem_atomics(0, 8192) for _ in range(3))
     peak_scatter = max(native.probe_smem_atomics(2, 8192) for _ in range(3))
     achieved = incr / (te_ms / 1e3)
     peaks = measured_peaks()
     hbm_peak = peaks.get("hbm_gbs")
     compulsory = G * x.shape[1] + (p1 - p0) * 4            # bins once + fp32 outputs
-    roofline = {"bound": "smem_atomic", "achieved": achieved / 1e9, "peak": peak_atomic / 1e9,
-                "unit": "Gincr/s", "frac": achieved / peak_atomic,
+    roofline = {"bound": "shared memory pipe", "achieved": achieved / 1e9,
+                "peak": peak_atomic / 1e9, "unit": "Gsamples/s", "frac": achieved / peak_atomic,
                 "traffic": profile_traffic(),
-                "note": "achieved = pairs x (T - tau) histogram increments per launch / mean "
-                        "launch time (CUDA events); peak = conflict-free shared-memory atomicAdd "
-                        "rate measured live by tenex_probe_smem_atomics (mode 0) on this GPU "
-                        "(MEASURED_PEAKS.json has no shared-memory-atomic figure)",
-                "scatter_peak": peak_scatter / 1e9,
-                "frac_of_scatter": achieved / peak_scatter,
-                "scatter_note": "second denominator, for context: the same probe with each lane "
-                                "adding into a random word of a 16 KB histogram (mode 2), the "
-                                "access pattern of a histogram of random cells",
-                "te_kernel_ms": te_ms}
+                "note": "achieved = pairs x (T - tau) samples per launch / mean launch time (CUDA "
+                        "events); peak = conflict-free shared-memory atomicAdd rate measured live "
+                        "by tenex_probe_smem_atomics (mode 0) on this GPU, one increment per "
+                        "sample. Pairs of few cells are contracted on the tensor cores without "
+                        "increments, so this compares the launch with counting every pair and is "
+                        "not a utilisation of either kernel; both are bound by the shared-memory "
+                        "pipe (load-store part 66% busy in the contraction, 61 to 75% in the "
+                        "counting: profiles/te_mma.md). traffic = DRAM bytes of both kernels",
+                "scatter_rate": peak_scatter / 1e9,
+                "times_scatter": achieved / peak_scatter,
+                "scatter_note": "the same probe with each lane adding into a random word of a 16 KB "
+                                "histogram (mode 2): what counting alone could reach at most on "
+                                "random cells; above 1 because of the contraction",
+                "te_launch_ms": te_ms}
     roofline_hbm = {"bound": "hbm", "achieved": compulsory / (te_ms / 1e3) / 1e9,
                     "peak": hbm_peak, "unit": "GB/s",
                     "frac": (compulsory / (te_ms / 1e3) / 1e9 / hbm_peak) if hbm_peak else None,
@@ -414,11 +418,12 @@ def _te_device_ms(kern, db, npv_t, bmax, reps: int = 3) -> float:
 
 def _smem_roofline(pairs: int, N: int, ms: float, peak: float) -> dict:
     achieved = pairs * N / (ms / 1e3)
-    return {"bound": "smem_atomic", "achieved": achieved / 1e9, "peak": peak / 1e9,
-            "unit": "Gincr/s", "frac": achieved / peak,
-            "note": "pairs x (T - tau) histogram increments / device time of the TE launch; "
-                    "peak = conflict-free shared-memory atomic probe (tenex_probe_smem_atomics "
-                    "mode 0) measured live"}
+    return {"bound": "shared memory pipe", "achieved": achieved / 1e9, "peak": peak / 1e9,
+            "unit": "Gsamples/s", "frac": achieved / peak,
+            "note": "pairs x (T - tau) samples / device time of the TE launch; peak = "
+                    "conflict-free shared-memory atomic probe (tenex_probe_smem_atomics mode 0) "
+                    "measured live, one increment per sample; pairs of few cells are contracted "
+                    "on the tensor cores without increments"}
 
 
 def cfg3_leg(dev, peak: float, with_cpu: bool = True) -> dict:

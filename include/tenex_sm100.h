@@ -90,10 +90,11 @@ size_t tenex_te_pairs_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 
 /* The same plus room for the tensor-core histograms of the all-pairs entry points, where
  * all pairs of n_vars genes are enough work for them: tables (about 5 KB a gene) and bit
- * planes (row_len / 4 bytes for each of a gene's bins up to 16, at most 8 GiB). With a smaller workspace (at least
- * tenex_te_pairs_workspace_bytes) they use what fits, down to none: every pair then
- * runs in the shared-memory kernel. The tables start at the workspace's next multiple
- * of 256 bytes; an aligned workspace wastes none of it. */
+ * planes (row_len / 4 bytes for each of a gene's bins up to 16, at most 8 GiB). With a
+ * smaller workspace (at least tenex_te_pairs_workspace_bytes) they use what fits if it is
+ * enough to be the faster; otherwise every pair runs in the shared-memory kernel. The
+ * tables start at the workspace's next multiple of 256 bytes; an aligned workspace wastes
+ * none of it. */
 size_t tenex_te_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 
 /* The launch shape the histogram kernels would use on the current device for
@@ -150,7 +151,8 @@ int tenex_te_pairfree_counts(const uint8_t* bins, int64_t ld, const int32_t* n_p
  * the call's outcome, written on `stream`: 0 = inputs valid and every pair
  * computed (also for an empty range), 1 = a bin value >= its gene's n_per_var
  * or n_per_var outside [1, b_max] (no TE computed), 3 = a work item's histogram
- * did not fit shared memory (its pairs not computed); NULL skips it.
+ * did not fit shared memory (its pairs not computed) or a device wait ran out
+ * (results invalid); NULL skips it.
  * Allocates nothing: no cudaMalloc, cudaFree or allocating library call. */
 int tenex_te_pairfree_static(const uint8_t* bins, int64_t ld, const int32_t* n_per_var,
                              int b_max, int n_vars, int64_t row_len, int64_t lag,

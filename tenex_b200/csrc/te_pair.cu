@@ -1477,7 +1477,8 @@ int static_scratch(void** out) {
 // Status word of a static-scratch call: 0 = inputs valid and every pair
 // computed; 1 = a bin value >= its gene's n_per_var or n_per_var outside
 // [1, b_max] (no TE computed); 3 = a work item's histogram did not fit shared
-// memory (its pairs were not computed).
+// memory (its pairs were not computed) or a wait of the tensor-core pipeline ran out
+// (results invalid).
 __global__ void static_status_kernel(const WsHeader* h, int32_t* status) {
   const int bad = h->bad_data;
   *status = bad != 0 ? bad : (h->bad_item != 0 ? 3 : 0);
