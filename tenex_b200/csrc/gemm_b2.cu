@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(B2Layout<TN>::kThreads, B2Layout<TN>::kCtasPer
     bool ok = true;
     uint32_t s = 0, ph = 0;
     for (int k = 0; k < nk; ++k) {
-      if (*(volatile int*)abort_flag || !mbar_wait(&full[s], ph)) {
+      if (__any_sync(0xffffffffu, *(volatile int*)abort_flag) || !mbar_wait_warp(&full[s], ph)) {
         ok = false;
         break;
       }

@@ -41,6 +41,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// mbar_wait by a whole, converged warp that goes on together: one answer for all lanes.
+// Lanes poll on their own, so at the limit some could give up where others do not, and
+// those would wait at the warp's next barrier for lanes that have left the loop.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+}
+
 // mbar_wait with a pause between polls, for warps that only wait (keeps them off
 // the shared-memory pipe while the producer's copies land); same bound on polls.
 __device__ __forceinline__ bool mbar_wait_sleep(uint64_t* bar, uint32_t parity, unsigned ns) {

@@ -865,7 +865,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
           vf1 = __ldg(Fk + of1);
           vq1 = __ldg(Pk + oq1);
         }
-        if (!mbar_wait(&S.empty[s], ph)) {
+        if (!mbar_wait_warp(&S.empty[s], ph)) {
           *(volatile int*)&S.abort = 1;
           break;
         }
@@ -890,7 +890,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2) te_mma_
       const uint32_t last = (uint32_t)(((M.N & 255) + 63) >> 6);  // MMAs of a short last step
       uint32_t s = stage, ph = parity;
       for (int k = 0; k < n_steps; ++k) {
-        if (!mbar_wait(&S.full[s], ph)) {
+        if (!mbar_wait_warp(&S.full[s], ph)) {
           *(volatile int*)&S.abort = 1;
           break;
         }
