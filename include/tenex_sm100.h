@@ -85,7 +85,9 @@ int tenex_device_query(int device, tenex_dev_info* info);
  * by bin count), rounded up to 256 bytes; plus, when pairs with b up to b_max
  * would not fit a shared-memory slot on the current device (coarsening off), the
  * global-memory histogram slots of the overflow launch. A workspace without them
- * makes such a call fail with the size it needs. */
+ * makes such a call fail with the size it needs. It may start at any multiple of 4
+ * bytes, of 8 where targets of so many bins keep their own tables in it (otherwise
+ * TENEX_ERR_BADARG). */
 size_t tenex_te_pairs_workspace_bytes(int n_vars, int64_t row_len, int b_max);
 
 /* The same plus room for the tensor-core histograms of the all-pairs entry points, where

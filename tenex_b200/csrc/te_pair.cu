@@ -1302,6 +1302,11 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
                   "pairs with b up to %d do not fit shared memory and need %lld bytes of "
                   "global-memory slots in the workspace (%lld given; size it with "
                   "tenex_te_workspace_bytes)", b_max, (long long)need, (long long)ws_bytes);
+    // the marginal tables hold 8-byte vectors, all else here words (gmarg_words is even)
+    if (marg_bytes && (reinterpret_cast<uintptr_t>(workspace) & 7))
+      return fail(TENEX_ERR_BADARG,
+                  "targets with b up to %d keep their tables in the workspace, which must be 8-byte "
+                  "aligned for them", b_max);
     unsigned char* g = reinterpret_cast<unsigned char*>(workspace) + ws_total(n, b_max);
     P.gslots = reinterpret_cast<uint32_t*>(g);
     if (marg_bytes) {
@@ -1345,7 +1350,8 @@ static int te_run(const uint8_t* bins, int64_t ld, const int32_t* npv, int b_max
   // pairs of few cells go to the tensor cores where the workspace has room for their
   // tables and bit planes (one sized by tenex_te_workspace_bytes has), which hold 16-byte
   // vectors and start at its next multiple of 256 bytes. The rest of the workspace holds
-  // whole words only, so callers may give it at any such address.
+  // whole words (but for the overflow launch's tables, above), so callers may give it at
+  // any such address.
   const int64_t skip = -(int64_t)(reinterpret_cast<uintptr_t>(wsb) + ws_used) & 255;
   if (!pairs && te_mma_layout(&M, wsb + ws_used + skip, (int64_t)ws_bytes - ws_used - skip))
     P.cut = M.cut;

@@ -407,3 +407,31 @@ def test_items_of_few_sources(cuda, n, b, T):
     bins, npv, bmax = O.remap(rng.integers(0, b, (n, T)).astype(np.int32))
     te = _gpu_te(bins, npv, bmax, cuda).cpu().numpy()
     assert np.max(np.abs(te - O.te_pairfree(bins, npv))) <= TOL
+
+
+def test_overflow_tables_need_an_8_byte_aligned_workspace(cuda):
+    """Targets of hundreds of bins keep 8-byte vectors in the workspace: at an odd word the call
+    is refused before any launch, at a multiple of 8 bytes it runs."""
+    rng = np.random.default_rng(9)
+    n, T, bmax = 3, 400, 250
+    bins, npv, b = O.remap(rng.integers(0, bmax, (n, T)).astype(np.int32))
+    db = D.pack_bins(bins, cuda)
+    npv_t = torch.as_tensor(npv, dtype=torch.int32, device=cuda)
+    P, s = n * (n - 1), native.stream_ptr()
+    nb = D.workspace(cuda, n, T, b).numel()
+    mem = torch.empty(nb + 8, dtype=torch.uint8, device=cuda)
+    out = torch.zeros(P, dtype=torch.float32, device=cuda)
+    for offset in (4, 8):
+        ws = mem[offset:offset + nb]
+        args = (db.ptr(), db.ld, npv_t.data_ptr(), b, n, T, 1, 0, P, out.data_ptr(),
+                native.OUT_PAIRFREE, 0, ws.data_ptr(), nb, None, s)
+        if offset % 8:
+            with pytest.raises(native.TenexError) as e:
+                native.call("tenex_te_pairfree", *args)
+            assert e.value.status == native.TENEX_ERR_BADARG and "8-byte" in str(e.value)
+            torch.cuda.synchronize()
+            assert not bool(out.any())
+        else:
+            native.call("tenex_te_pairfree", *args)
+            native.call("tenex_workspace_status", ws.data_ptr(), s)
+            assert np.max(np.abs(out.cpu().numpy() - O.te_pairfree(bins, npv, tau=1))) <= TOL
