@@ -109,7 +109,8 @@ __global__ void block_shuffle_kernel(const uint8_t* __restrict__ in, int64_t in_
 // per gene and group of `per` copies reads the row once. 16 output bytes then come from
 // at most two places of the row, five aligned words each, put together by funnel shifts
 // and merged at the block's end. 2,000 genes x 100 copies of 5,000 bytes (1 GB written):
-// 2.37 -> 1.09 ms; the kernel above gathers byte by byte from global memory.
+// 2.37 -> 1.09 ms (0.6 now), 1,000 x 100 of 500 bytes 89 -> 28 us; the kernel above gathers
+// byte by byte from global memory.
 constexpr uint32_t kShufflePad = 32;  // zero bytes before and after the row
 constexpr int kShuffleSmem = 100 * 1024;  // most shared memory of a CTA: two share an SM
 __global__ void __launch_bounds__(256) block_shuffle_row_kernel(
@@ -120,8 +121,15 @@ __global__ void __launch_bounds__(256) block_shuffle_row_kernel(
   const uint32_t* words = reinterpret_cast<const uint32_t*>(sh);
   const int g = blockIdx.x;
   const uint8_t* src = in + (int64_t)g * in_ld;
-  for (uint32_t i = threadIdx.x; i < row + 2 * kShufflePad; i += blockDim.x)
-    sh[i] = i >= kShufflePad && i < row + kShufflePad ? src[i - kShufflePad] : 0;
+  // 16 bytes at a time where the row's address allows it (a row of 100,000 bytes 20 us, 90
+  // byte by byte)
+  const uint32_t wide = reinterpret_cast<uintptr_t>(src) & 15 ? 0u : row & ~15u;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x * 16u; i < wide; i += blockDim.x * 16u)
+    *reinterpret_cast<uint4*>(sh + kShufflePad + i) =
+        __ldg(reinterpret_cast<const uint4*>(src + i));
+  for (uint32_t i = wide + threadIdx.x; i < row; i += blockDim.x) sh[kShufflePad + i] = src[i];
+  if (threadIdx.x < kShufflePad) sh[threadIdx.x] = sh[kShufflePad + row + threadIdx.x] = 0;
   __syncthreads();
   // 16 bytes of the row from byte j >= -16 on
   auto take = [&](int j, uint32_t (&w)[4]) {
@@ -136,7 +144,14 @@ __global__ void __launch_bounds__(256) block_shuffle_row_kernel(
     }
   };
   const int c0 = blockIdx.y * per, c1 = min(copies, c0 + per);
-  for (uint32_t i0 = threadIdx.x * 16u; i0 < row; i0 += blockDim.x * 16u) {
+  // a row shorter than 16 bytes a thread: `width` threads (a power of two) a copy, several
+  // copies at a time (1,000 genes x 100 copies of 500 bytes 114 us with one at a time)
+  const uint32_t pieces = (row + 15u) / 16u;
+  const uint32_t width = pieces >= blockDim.x ? blockDim.x
+                         : pieces > 1u       ? 1u << (32 - __clz(pieces - 1u))
+                                             : 1u;
+  const int first = c0 + (int)(threadIdx.x / width), step = (int)(blockDim.x / width);
+  for (uint32_t i0 = (threadIdx.x & (width - 1u)) * 16u; i0 < row; i0 += width * 16u) {
     const uint32_t b = i0 / blK, off = i0 - b * blK;
     const bool in1 = i0 < head;
     const uint32_t len = in1 ? min(16u, blK - off) : 16u;  // bytes of the first place
@@ -147,7 +162,7 @@ __global__ void __launch_bounds__(256) block_shuffle_row_kernel(
       const int k = (int)len - 4 * (int)u;  // of this word's bytes
       mask[u] = k >= 4 ? 0xffffffffu : k <= 0 ? 0u : (1u << (8 * k)) - 1u;
     }
-    for (int c = c0; c < c1; ++c) {
+    for (int c = first; c < c1; c += step) {
       const int32_t* pg = perm + (int64_t)c * perm_stride + (int64_t)g * n_blocks;
       uint32_t j = i0;
       if (in1) {
@@ -280,7 +295,15 @@ extern "C" int tenex_block_shuffle_many(const uint8_t* in, int64_t in_ld, int n_
   // several copies, rows that fit shared memory next to a second CTA, blocks of 16 bytes
   // or more (one copy: 10.8 us by the kernel above, 13.9 by this one, 1,000 x 5,000)
   const int64_t sh = row + 2 * kShufflePad;
-  if (n_copies > 1 && (int64_t)block_length * K >= 16 && sh <= kShuffleSmem) {
+  // the longer the row, the longer a CTA takes to bring it in (30,000 bytes 2 us, 100,000 12)
+  // and the more of them it takes that others hide that: (row / 3,700)^2, as measured (blocks
+  // of 50, us by this kernel / the one above: 100,000 bytes 10 genes x 2 copies 22 / 9, 30 x 4
+  // 24 / 20, 300 x 2 78 / 73, 10 x 100 105 / 113, 1,000 x 4 336 / 454; 30,000 bytes 10 x 2 9.9 /
+  // 9.1, 30 x 16 13 / 22). Rows at any byte come in byte by byte, so short ones only
+  const bool aligned = !((reinterpret_cast<uintptr_t>(in) | (uint64_t)in_ld) & 15);
+  const int64_t many = (row / 3700) * (row / 3700);
+  const bool enough = aligned ? (int64_t)n_vars * n_copies >= many : row <= 4096;
+  if (n_copies > 1 && (int64_t)block_length * K >= 16 && sh <= kShuffleSmem && enough) {
     DevAttr A;
     const int st = current_device_attr(&A);
     if (st) return st;

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from tenex_b200 import TransferEntropyEngine, workloads as W
+from tenex_b200 import TransferEntropyEngine, native, workloads as W
 from tenex_b200.inference import NetWeaver
 from tenex_b200.inference.surrogate_test import (SurrogateAccumulator, build_block_perm,
                                                  run_surrogates, surrogate_statistics)
@@ -272,3 +272,29 @@ def test_permutations_come_before_the_workspace(cuda, monkeypatch, kernel, hi, a
     s1, _, _ = ST.SurrogateTestMethod.accumulate(obs, cuda, bins.reshape(20, 300, 1), npv, bmax,
                                                  kernel, 1, 3, "block", 20, 5)
     assert order == asked and s1.any()
+
+
+@pytest.mark.parametrize("row", [17, 31, 33, 500, 2049, 4096, 4113, 30001, 32768, 32785, 102336,
+                                 102337])
+@pytest.mark.parametrize("n,S,bl,offset", [(3, 2, 16, 0), (2, 37, 17, 0), (5, 3, 16, 1),
+                                           (700, 3, 50, 0)])
+def test_row_shuffles_at_the_edges_of_their_ways(cuda, row, n, S, bl, offset):
+    """Rows shorter than a CTA's pieces (several copies at a time) and longer, rows at any byte,
+    lengths around the limits of the way through shared memory: bytes of a plain gather."""
+    if bl > row:
+        pytest.skip("block longer than the row")
+    g = torch.Generator(device=cuda).manual_seed(row + n)
+    ld = D.empty_bins(1, row, 1, cuda).ld + (offset and 3)
+    mem = torch.randint(0, 256, (n * ld + 64,), generator=g, device=cuda, dtype=torch.uint8)
+    src = mem[offset:offset + n * ld].view(n, ld)
+    nb = row // bl
+    perms = torch.argsort(torch.rand((S, n, nb), generator=g, device=cuda), dim=2).to(torch.int32)
+    out_ld = (row + 15) // 16 * 16
+    out = torch.full((S * n, out_ld), 7, dtype=torch.uint8, device=cuda)
+    native.call("tenex_block_shuffle_many", src.data_ptr(), ld, n, row, 1, perms.data_ptr(), S, nb,
+                bl, out.data_ptr(), out_ld, n * out_ld, native.stream_ptr())
+    idx = (perms.long()[..., None] * bl + torch.arange(bl, device=cuda)).view(S, n, nb * bl)
+    tail = torch.arange(nb * bl, row, device=cuda).expand(S, n, -1)
+    want = torch.gather(src[:, :row].expand(S, n, row), 2, torch.cat((idx, tail), 2))
+    got = out.view(S, n, out_ld)
+    assert torch.equal(got[..., :row], want) and bool((got[..., row:] == 7).all())
