@@ -108,9 +108,9 @@ __global__ void block_shuffle_kernel(const uint8_t* __restrict__ in, int64_t in_
 // The same with a gene's row in shared memory, for blocks of 16 bytes or more: one CTA
 // per gene and group of `per` copies reads the row once. 16 output bytes then come from
 // at most two places of the row, five aligned words each, put together by funnel shifts
-// and merged at the block's end. 2,000 genes x 100 copies of 5,000 bytes (1 GB written):
-// 2.37 -> 1.09 ms (0.6 now), 1,000 x 100 of 500 bytes 89 -> 28 us; the kernel above gathers
-// byte by byte from global memory.
+// and merged at the block's end. 1,000 genes x 100 copies of 5,000 bytes (0.5 GB written):
+// 0.59 -> 0.32 ms, of 500 bytes 89 -> 28 us; the kernel above gathers byte by byte from
+// global memory.
 constexpr uint32_t kShufflePad = 32;  // zero bytes before and after the row
 constexpr int kShuffleSmem = 100 * 1024;  // most shared memory of a CTA: two share an SM
 __global__ void __launch_bounds__(256) block_shuffle_row_kernel(
