@@ -93,9 +93,10 @@ os.register_at_fork(after_in_child=_forget_pool)
 
 def all_finite(a: np.ndarray) -> bool:
     """np.isfinite(a).all() for a large C-contiguous array, checked in one slab (of at
-    most 4M elements) per host copy thread (ufuncs run without the GIL)."""
+    most 4M elements) per host copy thread (ufuncs run without the GIL). us on the threads /
+    in one call: 1M elements 228 / 134, 2M 257 / 256, 3M 275 / 385, 8M 470 / 1,300."""
     a = np.asarray(a)
-    if a.size < (1 << 20) or not a.flags.c_contiguous:
+    if a.size < (5 << 19) or not a.flags.c_contiguous:
         return bool(np.isfinite(a).all())
     flat = a.reshape(-1)
     step = min(1 << 22, -(-flat.size // _copy_workers))

@@ -82,3 +82,31 @@ def test_permutations_are_sorted_one_by_one_when_memory_is_short(monkeypatch):
         torch.OutOfMemoryError("no room")))
     with pytest.raises(torch.OutOfMemoryError):
         build_block_perm(6, 400, "block", 10, 2, 9, 5, "cpu")
+
+
+@pytest.mark.parametrize("size", [1, (5 << 19) - 1, 5 << 19, (5 << 19) + 1, (1 << 22) + 3])
+def test_finite_check_around_the_size_where_threads_take_part(monkeypatch, size):
+    used = []
+    pool = D._pool()
+    monkeypatch.setattr(D, "_pool", lambda: (used.append(1), pool)[1])
+    a = np.zeros(size, np.float32)
+    assert D.all_finite(a) and bool(used) == (size >= 5 << 19)
+    for at in (0, size // 2, size - 1):
+        for bad in (np.nan, np.inf, -np.inf):
+            a[at] = bad
+            assert not D.all_finite(a)
+        a[at] = 0
+
+
+def test_finite_check_of_a_large_array_in_a_forked_process():
+    a = np.zeros(1 << 22, np.float32)
+    assert D.all_finite(a)
+    ready = threading.Barrier(D._copy_workers + 1)
+    tasks = [D._pool().submit(ready.wait, 20) for _ in range(D._copy_workers)]
+    ready.wait(20)
+    assert len([t.result() for t in tasks]) == D._copy_workers and D.all_finite(a)
+    pid = os.fork()
+    if pid == 0:
+        threading.Timer(20, os._exit, (3,)).start()
+        os._exit(0 if D.all_finite(a) else 2)
+    assert os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]) == 0
