@@ -1013,9 +1013,9 @@ bool takes_every_pair(int b_max, int N) {
 }
 
 // Whether a launch over `pairs` pairs is faster with the tensor-core path than in the
-// counting kernel alone, with room for its planes. The path adds two launches and the plan's serial chain (25 us at
-// the least), the planes of all n genes however few the pairs, and an item's chain of
-// N / 256 steps; where only some pairs are its own the counting kernel runs after it, with
+// counting kernel alone, with room for its planes. The path adds two launches and the plan's
+// serial chain (25 us at the least), the planes of all n genes however few the pairs, and an
+// item's chain of N / 256 steps; where only some pairs are its own the counting kernel runs after it, with
 // its own last round of items. The counting kernel takes pairs x (N + about 2,000) / 2.1e12
 // s where its items (32 sources of one target at the least) fill the SMs; up to 17 genes
 // the two chains are about equally long. Measured, us with the path / without, b_max 6 | b_max 16:
@@ -1026,12 +1026,18 @@ bool takes_every_pair(int b_max, int N) {
 //   10 x 1,000,000 1,320 / 1,140 | 3,570 / 2,020   20 x 1,000,000 1,530 / 2,200 | 5,230 / 3,460
 //   10,000 x 20,000, b_max 16, one target's pairs 1,010 / 204, 16 targets' 1,960 / 1,750,
 //   32 targets' 2,900 / 3,180; 2,000 x 20,000, b_max 6, 1 target 182 / 79, 8: 197 / 221.
-// Over 700 sizes (2 to 10,000 genes, 100 to 1,000,000 samples) the choice is on average
-// within 1% of the better one.
+// Above 16 bins most genes usually have fewer (a bin count of 38 after coarsening comes from a
+// few), so the path takes most pairs there and is worth it sooner: 283 genes x 5,516 samples
+// of 3 bins, 3% of 38, 246 / 377; 311 x 3,714, 4 bins and 8% of 38, 322 / 454.
+// Over 2,700 sizes about the line (12 to 1,000 genes, 200 to 120,000 samples, with and without
+// genes of 38 bins) the choice is on average within 1.2% of the better one, and at most 28%
+// slower than the path always taken (one in ninety over 10%).
 bool worth_it(int n, int N, int b_max, int64_t pairs) {
   const double work = (double)pairs * (N + 2000.0), planes = (double)n * N;
-  if (!takes_every_pair(b_max, N))
-    return work >= 1e8 + std::min(1.5e5 * N, 5e8) + 25.0 * planes;
+  if (!takes_every_pair(b_max, N)) {
+    const double more = b_max > kMaxTgtBins ? std::min(2e4 * N, 7e8) : std::min(1.5e5 * N, 5e8);
+    return work >= 1e8 + more + 25.0 * planes;
+  }
   const double items = ((double)pairs / (n - 1) + 1) * ((n + 31) / 32), sms = 148;
   return pairs >= 300 && work * std::max(1.0, sms / items) >= 1e8 + 5.0 * planes;
 }

@@ -110,3 +110,14 @@ def test_finite_check_of_a_large_array_in_a_forked_process():
         threading.Timer(20, os._exit, (3,)).start()
         os._exit(0 if D.all_finite(a) else 2)
     assert os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]) == 0
+
+
+def test_workspace_has_the_tables_where_a_few_genes_have_many_bins():
+    """A bin limit above 16 mostly comes from a few genes: the tensor-core path is worth it for
+    smaller problems than at a limit of 16."""
+    L = native.lib()
+    for n, T in ((283, 5516), (311, 3714), (230, 1775)):
+        least = L.tenex_te_pairs_workspace_bytes(n, T, 38)
+        assert L.tenex_te_workspace_bytes(n, T, 38) > least + n * T // 8
+        least = L.tenex_te_pairs_workspace_bytes(n, T, 16)
+        assert L.tenex_te_workspace_bytes(n, T, 16) < least + 256
