@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from tenex_b200 import TransferEntropyEngine, native, workloads as W
+from tenex_b200 import TransferEntropyEngine, workloads as W
 from tenex_b200.inference import NetWeaver
 from tenex_b200.inference.surrogate_test import (SurrogateAccumulator, build_block_perm,
                                                  run_surrogates, surrogate_statistics)
@@ -281,6 +281,7 @@ def test_permutations_come_before_the_workspace(cuda, monkeypatch, kernel, hi, a
 def test_row_shuffles_at_the_edges_of_their_ways(cuda, row, n, S, bl, offset):
     """Rows shorter than a CTA's pieces (several copies at a time) and longer, rows at any byte,
     lengths around the limits of the way through shared memory: bytes of a plain gather."""
+    from tenex_b200 import native
     if bl > row:
         pytest.skip("block longer than the row")
     g = torch.Generator(device=cuda).manual_seed(row + n)
